@@ -71,6 +71,7 @@ struct MarchArgs {
     // that are redone); ftab is null for face-independent coefficients
     const double* ftab;
     CoefPtrs cp;
+    long long n_cols;  // Nu x Nw x NV
 };
 
 // Row of the per-face table (doubles per face; 224 bytes, a multiple of 16).
@@ -1747,6 +1748,7 @@ inline MarchArgs make_march_args(const SweepGeom& g, const void* in, void* vL, v
     a.oV = g.ns * g.c1 * g.c2;
     a.NV = (int)g.nv;
     a.n_ut = (a.Nu + 31) / 32;
+    a.n_cols = g.cols;
     if (!ucf) return a;  // face-dependent coefficients: the caller sets ftab and cp
     for (int q = 0; q < 56; ++q) a.ucf[q] = ucf[q];
     if (order == 3) {

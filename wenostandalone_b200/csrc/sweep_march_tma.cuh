@@ -38,6 +38,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -70,6 +72,14 @@ constexpr int kTmaOut = WSB_MTMA_OUTBUF;
 #endif
 constexpr int kPfStages = WSB_MTMA_PF_STAGES;
 constexpr int kPfOut = WSB_MTMA_PF_OUTBUF;
+// Single sweeps with plain stores: their per-lane copies and stores go
+// through L1, which gets what shared memory leaves (a fourth stage cost 9%
+// at 200^3 x 8); the previous chunk's face states stay in the other output
+// tile for the rows whose 32-byte sectors straddle two chunks.
+constexpr int kPstStages = 3;
+constexpr int kPstOut = 2;
+__host__ __device__ constexpr int mtma_stages(bool pf, bool pst) { return pst ? kPstStages : (pf ? kPfStages : kTmaStages); }
+__host__ __device__ constexpr int mtma_outs(bool pf, bool pst) { return pst ? kPstOut : (pf ? kPfOut : kTmaOut); }
 // rows f0 .. f0 + 8 of a chunk (WENO5 / WENO7 table rows)
 __host__ __device__ constexpr int pf_row_doubles(int order) {
     return order == 7 ? kFaceRow7 : (order == 3 ? kFaceRow3 : kFaceRow);
@@ -187,7 +197,7 @@ struct MtmaSlot {
     const MtmaEntry* e;
 };
 static_assert(sizeof(MtmaItemArgs) % 8 == 0 && sizeof(MtmaSlot) <= 256, "per-warp argument slot");
-constexpr int kMtmaSlot = 256;  // bytes of shared memory per warp for the item's arguments
+constexpr int kMtmaSlot = 256;  // bytes of shared memory per warp for the item's arguments (or 32 offsets)
 inline MtmaGeo mtma_geo(const MarchArgs& a) {
     MtmaGeo g{};
     g.in = a.in; g.vL = a.vL; g.vR = a.vR;
@@ -220,7 +230,11 @@ __device__ __forceinline__ const auto& mtma_geo_of(const MarchArgs& a, const Mtm
 // entry); each item finds its entry, whose geometry, maps, loader (TMA or
 // per lane) and store kind (TMA or plain) it uses, with the coefficients of
 // the kernel's MarchArgs.
-template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER, int WS, bool MULTI>
+// PST (single sweeps): per-lane loads and plain stores, compiled in.  A lane
+// may then hold any column, so the tiles run over the columns of all cross
+// axes in turn (u fastest, then w, v) and only the sweep's last tile has
+// idle lanes.
+template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER, int WS, bool MULTI, bool PST = false>
 __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CUtensorMap* toutL0,
                                                const CUtensorMap* toutR0, const MarchArgs& a, const MarchTmaArgs& t,
                                                const MtmaEntry* __restrict__ ents,
@@ -229,8 +243,8 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     static_assert(WS == 0 || WS == 3 || (ORDER == 5 && sizeof(T) == 8),
                   "mapped / Z weights: the FP64 WENO5 engine");
     static_assert(WS != 1 || !PF, "mapped weights: face-independent coefficients");
-    constexpr int F = kTmaF, S = PF ? kPfStages : kTmaStages;
-    constexpr int NOUT = PF ? kPfOut : kTmaOut;             // output tiles per warp
+    constexpr int F = kTmaF, S = mtma_stages(PF, PST);
+    constexpr int NOUT = mtma_outs(PF, PST);                // output tiles per warp
     constexpr unsigned OB = 32u * F * sizeof(T);          // one output array tile
     constexpr int XW = sizeof(T) == 8 ? 34 : 36;          // KIND 1 tile width
     constexpr int XS = sizeof(T) == 8 ? 1 : 3;            // KIND 1 column of lane 0
@@ -254,7 +268,8 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     unsigned char* obuf = wbase;
     unsigned char* ring = wbase + t.ring_off;
     unsigned long long* bars = (unsigned long long*)(base + (size_t)kTmaWarps * warp_bytes) + warp * S;
-    // grouped sweeps: the warp's argument slot, after the mbarriers
+    // after the mbarriers: the warp's argument slot (grouped sweeps), or its
+    // columns' offsets in the face arrays (PST)
     MtmaSlot* slot = (MtmaSlot*)(base + (size_t)kTmaWarps * warp_bytes + (size_t)kTmaWarps * S * 8 +
                                  (size_t)warp * kMtmaSlot);
     if (lane == 0) {
@@ -340,15 +355,19 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         auto mapL = [&]() { return MULTI ? &slot->e->toutL : toutL0; };
         auto mapR = [&]() { return MULTI ? &slot->e->toutR : toutR0; };
         const bool ldr = MULTI ? te.ldr != 0 : LDR == 1;
-        // plain stores (face rows not 16-byte multiples): grouped sweeps only
-        // (the single-sweep kernels keep their registers for the face body)
-        const bool pst = MULTI && te.pst != 0;
+        // plain stores (face rows not 16-byte multiples): per entry in grouped
+        // sweeps, a kernel of its own for a single sweep (as a branch beside
+        // the TMA stores it cost the face body two registers and a spill)
+        const bool pst = MULTI ? te.pst != 0 : PST;
         T* __restrict__ outL = (T*)g.vL;
         T* __restrict__ outR = (T*)g.vR;
         // faces written: the core faces 3 .. ns-4 (chunks from face 4, face 3 by
         // the prologue), or every face 0 .. ns-1 for WENO3 (chunks from face 0)
         const int o_last = ORDER == 3 ? (int)g.ns : (int)g.ns - 3;  // one past the last face
-        auto column = [&](int u0, int wv, int vv) {
+        const T* colp = nullptr;   // PST: this lane's column
+        bool live = false;         // the lane holds a column of the sweep
+        auto column = [&](int u0, int wv, int vv) -> const T* {
+            if constexpr (PST) return colp;
             const int uc = u0 + lane < g.Nu ? u0 + lane : g.Nu - 1;
             return (const T*)g.in + g.in_off + uc * g.sU + wv * g.sW + vv * g.sV;
         };
@@ -372,7 +391,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 unsigned char* tp = tile_ptr(k);
                 const long long ncell = g.ns + 6;
                 const T* col = column(u0, w, v);
-                if (ORDER == 3 && KIND == 0 && sizeof(T) == 4 && te.ldr8) {
+                if (!PST && ORDER == 3 && KIND == 0 && sizeof(T) == 4 && te.ldr8) {
                     // WENO3 (latency-bound, few registers): the warp copies
                     // the tile together in 8-byte pairs.  In copy k, lane l
                     // takes pair l % 4 of column l / 4 + 8k, so one
@@ -420,6 +439,14 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                                      : "memory");
                     }
                 }
+                if constexpr (PF && LDR == 1) {
+                    // rows J0 .. J0 + 8, shared by the lanes (wait_tile syncs the warp)
+                    const unsigned char* src = (const unsigned char*)row(J0);
+                    const unsigned dst = smem_u32(srow(k, 0));
+                    for (int q = lane * 16; q < RB; q += 32 * 16)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + q), "l"(src + q)
+                                     : "memory");
+                }
                 asm volatile("cp.async.commit_group;\n" ::: "memory");
             }
         };
@@ -436,7 +463,9 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 else if (after == 1) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
                 else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
                 // the cooperative WENO3 loader fills rows that other lanes read
-                if (ORDER == 3 && KIND == 0 && sizeof(T) == 4 && te.ldr8) __syncwarp();
+                if (!PST && ORDER == 3 && KIND == 0 && sizeof(T) == 4 && te.ldr8) __syncwarp();
+                // as does the copy of the per-face table rows
+                if (PF && LDR == 1) __syncwarp();
             }
             n_waited = k + 1;
             return true;
@@ -444,11 +473,28 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
 
         const int sg = (int)(li % g.n_seg);
         long long tt = li / g.n_seg;
-        const int ut = (int)(tt % g.n_ut);
-        tt /= g.n_ut;
-        const int wv = (int)(tt % g.Nw);
-        const int vv = (int)(tt / g.Nw);
-        const int u0 = ut * 32;
+        int u0 = 0, wv = 0, vv = 0;
+        int c_end = 32;            // PST: columns of this tile
+        long long* offs = (long long*)slot;
+        if constexpr (PST) {
+            const long long c0 = tt * 32;
+            live = c0 + lane < a.n_cols;
+            c_end = a.n_cols - c0 < 32 ? (int)(a.n_cols - c0) : 32;
+            tt = live ? c0 + lane : a.n_cols - 1;  // idle lanes shadow the last column
+            const long long u = tt % g.Nu;
+            tt /= g.Nu;
+            const long long w = tt % g.Nw, v = tt / g.Nw;
+            colp = (const T*)g.in + g.in_off + u * g.sU + w * g.sW + v * g.sV;
+            // (every lane's reads of the previous item's offsets ended before
+            // its last sync; the first chunk's stores sync after this write)
+            offs[lane] = u * g.oU + w * g.oW + v * g.oV;
+        } else {
+            u0 = (int)(tt % g.n_ut) * 32;
+            tt /= g.n_ut;
+            wv = (int)(tt % g.Nw);
+            vv = (int)(tt / g.Nw);
+            live = u0 + lane < g.Nu;
+        }
         const int f_start = (ORDER == 3 ? 0 : 4) + sg * g.seg;    // 4 mod 8 (WENO3: 0 mod 8)
         int f_end = f_start + g.seg;
         if (f_end > o_last) f_end = o_last;
@@ -506,8 +552,9 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 else if constexpr (ORDER == 7) march7_redo<MPF>(ga(), column(u0, wv, vv), 3, L, R);
                 else march_redo<MPF, PF>(ga(), column(u0, wv, vv), 3, L, R);
             }
-            if (u0 + lane < g.Nu) {
-                const long long oi = 3 + (long long)(u0 + lane) * g.oU + wv * g.oW + vv * g.oV;
+            if (live) {
+                const long long oi =
+                    3 + (PST ? offs[lane] : (long long)(u0 + lane) * g.oU + wv * g.oW + vv * g.oV);
                 outL[oi] = L;
                 outR[oi] = R;
             }
@@ -542,7 +589,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             // faces' arithmetic overlaps it.  A chunk of plain stores waits
             // for every store in flight (grouped sweeps: the last bulk store
             // may be the one from this buffer)
-            const bool wait_out = n_chunks >= (unsigned)NOUT;
+            const bool wait_out = !PST && n_chunks >= (unsigned)NOUT;
             if (NOUT > 1 && wait_out) {
                 if (lane == 0) {
                     if (MULTI && pst) bulk_wait_read0();
@@ -630,7 +677,60 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                     *(T*)(ob + OB + swz<T>((unsigned)lane, (unsigned)i)) = R;
                 }
             }
-            if (pst) {
+            if constexpr (PST) {
+                // plain stores: each row's run of 8 faces starts at a 32-byte
+                // sector, sh < SA faces before the chunk, and leaves as 16-byte
+                // stores; a segment's first and last chunks store face by face
+                // (the last one also what is left).  Runs cut at the chunk
+                // wrote two partial sectors each: 145 against 119 us for the
+                // y sweep of 134 (even) and 133 (odd) core faces, 128^2 x 5.
+                constexpr int SA = 32 / (int)sizeof(T), LR = F / G;  // LR lanes per row
+                const unsigned char* pv = obuf + (size_t)((n_chunks + 1) % NOUT) * (2 * OB);
+                const unsigned al = (unsigned)((uintptr_t)outL / sizeof(T)) + (unsigned)f0;
+                __syncwarp();
+                if (c > 0 && c < nch - 1 && (((uintptr_t)outL ^ (uintptr_t)outR) & 15) == 0) {
+                    T* const pL = outL + f0;
+                    T* const pR = outR + f0;
+#pragma unroll
+                    for (int k = 0; k < LR; ++k) {
+                        const unsigned cc = (unsigned)(lane / LR + (32 / LR) * k);
+                        if ((int)cc >= c_end) break;
+                        const long long off = offs[cc];
+                        const int rel = (lane % LR) * G - (int)((al + (unsigned)off) & (SA - 1));
+                        T x[G], y[G];
+#pragma unroll
+                        for (int q = 0; q < G; ++q) {
+                            const unsigned char* src =
+                                (rel + q < 0 ? pv : ob) + swz<T>(cc, (unsigned)(rel + q) & (F - 1));
+                            x[q] = *(const T*)src;
+                            y[q] = *(const T*)(src + OB);
+                        }
+                        if constexpr (sizeof(T) == 8) {
+                            *(double2*)(pL + (off + rel)) = make_double2(x[0], x[1]);
+                            *(double2*)(pR + (off + rel)) = make_double2(y[0], y[1]);
+                        } else {
+                            *(float4*)(pL + (off + rel)) = make_float4(x[0], x[1], x[2], x[3]);
+                            *(float4*)(pR + (off + rel)) = make_float4(y[0], y[1], y[2], y[3]);
+                        }
+                    }
+                } else {
+                    const int fi = lane & (F - 1), lo = f_start - f0, n_run = c == nch - 1 ? 2 * F : F;
+#pragma unroll 1
+                    for (int fb = fi; fb < n_run; fb += F) {
+#pragma unroll 1
+                        for (int cc = lane / F; cc < c_end; cc += 32 / F) {
+                            const long long off = offs[cc];
+                            const int rel = fb - (int)((al + (unsigned)off) & (SA - 1));  // face f0 + rel
+                            if (rel >= lo && rel < nF) {
+                                const unsigned char* src =
+                                    (rel < 0 ? pv : ob) + swz<T>((unsigned)cc, (unsigned)rel & (F - 1));
+                                outL[off + f0 + rel] = *(const T*)src;
+                                outR[off + f0 + rel] = *(const T*)(src + OB);
+                            }
+                        }
+                    }
+                }
+            } else if (pst) {
                 // plain stores: lane l writes face f0 + l % 8 of columns
                 // l / 8, l / 8 + 4, ..., so one instruction writes four
                 // columns' runs of 8 consecutive faces
@@ -639,18 +739,18 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 if (fi < nF) {
                     // (a rolled loop with one running index: unrolled, its
                     // addresses took 24 registers of the face body)
-                    const int c_end = g.Nu - u0 < 32 ? g.Nu - u0 : 32;
+                    const int u_end = g.Nu - u0 < 32 ? g.Nu - u0 : 32;
                     const long long step = (long long)(32 / F) * g.oU;
                     long long oi = (long long)(f0 + fi) + (long long)(u0 + lane / F) * g.oU + wv * g.oW + vv * g.oV;
 #pragma unroll 1
-                    for (int cc = lane / F; cc < c_end; cc += 32 / F, oi += step) {
+                    for (int cc = lane / F; cc < u_end; cc += 32 / F, oi += step) {
                         outL[oi] = *(const T*)(ob + swz<T>((unsigned)cc, (unsigned)fi));
                         outR[oi] = *(const T*)(ob + OB + swz<T>((unsigned)cc, (unsigned)fi));
                     }
                 }
             } else {
                 const int i_last = ORDER == 3 ? -1 : o_last - 1 - f0;  // the last core face, when in this chunk
-                if (i_last >= 0 && i_last < F && u0 + lane < g.Nu) {
+                if (i_last >= 0 && i_last < F && live) {
                     // outside the store map's extent (see plan_march_tma)
                     const long long oi = (o_last - 1) + (long long)(u0 + lane) * g.oU + wv * g.oW + vv * g.oV;
                     outL[oi] = *(const T*)(ob + swz<T>((unsigned)lane, (unsigned)i_last));
@@ -701,12 +801,12 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                                                    : (sizeof(T) == 8 ? WSB_MTMA_MIN_BLOCKS : WSB_MTMA_MIN_BLOCKS_F32))
 
 // One sweep: maps and arguments in the parameter bank.
-template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER = 5, int WS = 0>
+template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER = 5, int WS = 0, bool PST = false>
 __global__ void WSB_MTMA_BOUNDS(ORDER, T)
     sweep_march_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap toutL,
                            const __grid_constant__ CUtensorMap toutR, const __grid_constant__ MarchArgs a,
                            const MarchTmaArgs t) {
-    march_tma_body<MPF, KIND, T, LDR, PF, ORDER, WS, false>(&tin, &toutL, &toutR, a, t, nullptr, nullptr, 0,
+    march_tma_body<MPF, KIND, T, LDR, PF, ORDER, WS, false, PST>(&tin, &toutL, &toutR, a, t, nullptr, nullptr, 0,
                                                               a.n_items);
 }
 
@@ -741,8 +841,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32,
 // states leave by TMA stores when the face rows (ns elements) are 16-byte
 // multiples from 16-byte aligned bases, else by plain stores from the same
 // staging tiles.  seg_faces > 0 cuts every column into segments of about
-// that many faces; 0 sizes the segments to fill `sms` SMs about eight
-// work items per resident warp.  Returns 1003 (unsupported) for sweeps of
+// that many faces; 0 sizes the segments for `sms` SMs (march_segments).  Returns 1003 (unsupported) for sweeps of
 // fewer than 8 faces, a lane axis the march arguments did not choose, or a
 // missing driver entry point.
 struct MtmaPlan {
@@ -751,6 +850,56 @@ struct MtmaPlan {
     MarchTmaArgs t;
     size_t smem;
 };
+
+// Cut every column's faces (from face 4, WENO3 from face 0) into segments
+// of a multiple of 8 faces, one work item each.  seg_faces > 0: segments of
+// about that many faces.  0: the cut for which the `warps` resident warps,
+// taking the items in turn, are done first -- rounds x (faces of a segment
+// + the item's fixed cost, counted in faces: the wait for its first tile and
+// the window's start, and with plain stores the first and last chunks' stores
+// face by face).  A last round that is not full runs faster
+// (fewer warps share an SM), so rounds is the mean of items / warps and of
+// that rounded up; of cuts within 3% the finer.
+constexpr int kTmaItemFaces = 4, kPstItemFaces = 16;
+inline void march_segments(MarchArgs& a, int order, bool pst, long long seg_faces, long long warps) {
+    const long long chunks = ((order == 3 ? a.ns : a.ns - 7) + kTmaF - 1) / kTmaF;
+    const long long cols = pst ? (a.n_cols + 31) / 32 : (long long)a.n_ut * a.Nw * a.NV;
+    double best = -1.0;
+    for (long long n = 1; n <= chunks; ++n) {
+        const long long c = (chunks + n - 1) / n;          // chunks of a segment
+        if (n > 1 && c == (chunks + n - 2) / (n - 1)) continue;
+        if (seg_faces > 0) {
+            // the fewest segments of at most seg_faces faces (at least one chunk)
+            a.seg = (int)(c * kTmaF);
+            if (a.seg <= seg_faces) break;
+            continue;
+        }
+        const long long nseg = (chunks + c - 1) / c;
+        const double exact = (double)(cols * nseg) / (double)warps;
+        const double cost = 0.5 * (exact + std::ceil(exact)) * (double)(c * kTmaF + (pst ? kPstItemFaces : kTmaItemFaces));
+        if (best < 0.0 || cost < 1.03 * best) {
+            best = best < 0.0 ? cost : std::min(best, cost);
+            a.seg = (int)(c * kTmaF);
+        }
+    }
+    a.n_seg = (int)((chunks * kTmaF + a.seg - 1) / a.seg);
+    a.n_items = cols * a.n_seg;
+}
+
+// Shared-memory layout of the plan's kernel (pst: the single-sweep kernels
+// with plain stores).
+template <typename T>
+void march_layout(MtmaPlan& P, int order, bool pst) {
+    MarchTmaArgs& t = P.t;
+    const bool pf = P.a.ftab != nullptr;
+    const int nst = mtma_stages(pf, pst);
+    const int out_bytes = mtma_outs(pf, pst) * 2 * 32 * kTmaF * (int)sizeof(T);
+    t.ring_off = out_bytes;
+    t.rows_off = out_bytes + nst * t.stage_bytes;
+    t.warp_bytes = ((t.rows_off + (pf ? nst * pf_chunk_bytes(order) : 0) + 1023) / 1024) * 1024;
+    P.smem = 1024 + (size_t)kTmaWarps * t.warp_bytes + (size_t)kTmaWarps * nst * 8 +
+             (pst ? (size_t)kTmaWarps * kMtmaSlot : 0);
+}
 
 template <typename T>
 int plan_march_tma(const long long E[3], const SweepGeom& g, int dir, bool folded, const T* in, T* vL, T* vR,
@@ -836,173 +985,83 @@ int plan_march_tma(const long long E[3], const SweepGeom& g, int dir, bool folde
         t.pst = 0;
     // the lane axis must be the one the march arguments chose
     if ((t.kind == 1) != (a.sU == 1)) return 1003;
-    // segments over faces [4, ns-3), a multiple of 8 faces each
-    const long long nf4 = order == 3 ? g.ns : g.ns - 7;  // faces in the chunked range
-    const long long cols = (long long)a.n_ut * a.Nw * a.NV;
-#ifndef WSB_MTMA_ITEMS_PER_WARP
-#define WSB_MTMA_ITEMS_PER_WARP 8  // target work items per resident warp (200^3: two segments per column)
-#endif
-    long long nseg;
-    if (seg_faces > 0) {
-        nseg = (nf4 + seg_faces - 1) / seg_faces;
-    } else {
-        const long long want = (long long)sms * kTmaWarps * 3 * WSB_MTMA_ITEMS_PER_WARP;
-        nseg = (want + cols - 1) / cols;
-    }
-    const long long max_seg = (nf4 + kTmaF - 1) / kTmaF;
-    if (nseg > max_seg) nseg = max_seg;
-    if (nseg < 1) nseg = 1;
-    long long seg = (nf4 + nseg - 1) / nseg;
-    seg = ((seg + kTmaF - 1) / kTmaF) * kTmaF;
-    a.seg = (int)seg;
-    a.n_seg = (int)((nf4 + seg - 1) / seg);
-    a.n_items = cols * a.n_seg;
-    const bool pf = a.ftab != nullptr;
-    const int nst = pf ? kPfStages : kTmaStages;
-    const int out_bytes = (pf ? kPfOut : kTmaOut) * 2 * 32 * kTmaF * ES;
-    t.ring_off = out_bytes;
-    t.rows_off = out_bytes + nst * t.stage_bytes;
-    t.warp_bytes = ((t.rows_off + (pf ? nst * pf_chunk_bytes(order) : 0) + 1023) / 1024) * 1024;
-    P.smem = 1024 + (size_t)kTmaWarps * t.warp_bytes + (size_t)kTmaWarps * nst * 8;
+    march_segments(a, order, false, seg_faces, (long long)sms * kTmaWarps * 3);
+    march_layout<T>(P, order, false);
     return 0;
 }
 
-// One sweep.  Returns 1003 (unsupported) as plan_march_tma, for face rows
-// that are not 16-byte multiples, or for a per-face table whose field does
-// not suit TMA; the caller then uses another kernel.
+// Kernel of one sweep, by storage T, order and weights WS: [mp][kind1][path],
+// paths 0 TMA tiles in and out, 1 per-lane loads and TMA stores, 2 per-lane
+// loads and plain stores.  Per-lane loads read any alignment, so path 2
+// serves every layout the others refuse.  PF: with the per-face table, whose
+// kernels load by TMA (path 0) or take path 2.
+using MtmaFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, MarchTmaArgs);
+template <typename T, bool PF, int ORDER, int WS, bool MPF, int KIND>
+MtmaFn mtma_path(int path) {
+    if constexpr (KIND == 0 || sizeof(T) == 8) {
+        if (path == 2) return sweep_march_tma_kernel<MPF, KIND, T, 1, PF, ORDER, WS, true>;
+    }
+    if constexpr (!PF) {
+        if (path == 1) return sweep_march_tma_kernel<MPF, KIND, T, 1, false, ORDER, WS>;
+    }
+    return path == 0 ? sweep_march_tma_kernel<MPF, KIND, T, 0, PF, ORDER, WS> : nullptr;
+}
+template <typename T, bool PF, int ORDER, int WS>
+MtmaFn mtma_pick(bool mp, bool kind1, int path) {
+    if (mp) return kind1 ? mtma_path<T, PF, ORDER, WS, true, 1>(path) : mtma_path<T, PF, ORDER, WS, true, 0>(path);
+    return kind1 ? mtma_path<T, PF, ORDER, WS, false, 1>(path) : mtma_path<T, PF, ORDER, WS, false, 0>(path);
+}
+// ws: 0 JS, 1 mapped, 2 Z, 3 TENO; null for what no engine covers (mapped
+// and Z weights: FP64 WENO5, mapped without a table; WENO3: JS; per-face
+// tables: FP64)
+template <typename T>
+MtmaFn mtma_kernel(int order, int ws, bool pf, bool mp, bool kind1, int path) {
+    constexpr bool D = sizeof(T) == 8;
+    if (pf) {
+        if constexpr (D) {
+            if (order == 3) return ws == 0 ? mtma_pick<T, true, 3, 0>(mp, kind1, path) : nullptr;
+            if (order == 7)
+                return ws == 0 ? mtma_pick<T, true, 7, 0>(mp, kind1, path)
+                               : (ws == 3 ? mtma_pick<T, true, 7, 3>(mp, kind1, path) : nullptr);
+            return ws == 0 ? mtma_pick<T, true, 5, 0>(mp, kind1, path)
+                           : (ws == 2 ? mtma_pick<T, true, 5, 2>(mp, kind1, path)
+                                      : (ws == 3 ? mtma_pick<T, true, 5, 3>(mp, kind1, path) : nullptr));
+        }
+        return nullptr;
+    }
+    if (order == 3) return ws == 0 ? mtma_pick<T, false, 3, 0>(mp, kind1, path) : nullptr;
+    if (order == 7)
+        return ws == 0 ? mtma_pick<T, false, 7, 0>(mp, kind1, path)
+                       : (ws == 3 ? mtma_pick<T, false, 7, 3>(mp, kind1, path) : nullptr);
+    if (ws == 0) return mtma_pick<T, false, 5, 0>(mp, kind1, path);
+    if (ws == 3) return mtma_pick<T, false, 5, 3>(mp, kind1, path);
+    if constexpr (D) return ws == 1 ? mtma_pick<T, false, 5, 1>(mp, kind1, path) : mtma_pick<T, false, 5, 2>(mp, kind1, path);
+    return nullptr;
+}
+
+// One sweep.  Returns 1003 (unsupported) as plan_march_tma, or where no
+// kernel covers the weights; the caller then uses another kernel.
 template <typename T>
 int launch_march_tma(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, const T* in, T* vL,
                      T* vR, const MarchArgs& a0, cudaStream_t st, int sms, int order = 5, int ws = 0) {
     MtmaPlan P;
     const int prc = plan_march_tma<T>(E, g, dir, folded, in, vL, vR, a0, sms, order, 0, P);
     if (prc) return prc;
-    // face rows that are not 16-byte multiples: the grouped kernel's plain
-    // stores (batches), other kernels here
-    if (P.t.pst) return 1003;
     const MarchArgs& a = P.a;
     const MarchTmaArgs& t = P.t;
-    const bool kind1 = t.kind == 1;
-    const int ldr = t.ldr;
+    // face rows that are not 16-byte multiples leave by plain stores; so do
+    // the per-face kernels' when the field's rows do not suit TMA
+    const bool pf = a.ftab != nullptr;
+    const int path = t.pst || (pf && t.ldr) ? 2 : t.ldr;
+    const MtmaFn kfn = mtma_kernel<T>(order, ws, pf, mp, t.kind == 1, path);
+    if (!kfn) return 1003;
+    if (path == 2) march_layout<T>(P, order, true);
     const size_t smem = P.smem;
-    using KFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, MarchTmaArgs);
-    static const KFn table[2][2][2] = {
-        {{sweep_march_tma_kernel<false, 0, T, 0, false>, sweep_march_tma_kernel<false, 0, T, 1, false>},
-         {sweep_march_tma_kernel<false, 1, T, 0, false>, sweep_march_tma_kernel<false, 1, T, 1, false>}},
-        {{sweep_march_tma_kernel<true, 0, T, 0, false>, sweep_march_tma_kernel<true, 0, T, 1, false>},
-         {sweep_march_tma_kernel<true, 1, T, 0, false>, sweep_march_tma_kernel<true, 1, T, 1, false>}}};
-    KFn kfn = table[mp ? 1 : 0][kind1 ? 1 : 0][ldr];
-    const bool teno = ws == 3;
-    if ((ws == 1 || ws == 2) && (order != 5 || sizeof(T) != 8 || (ws == 1 && a.ftab))) return 1003;
-    if (ws == 2 && a.ftab) {
-        // WENO5-Z with the per-face table: FP64 with TMA input tiles
-        if constexpr (sizeof(T) == 8) {
-            if (ldr) return 1003;
-            static const KFn ptablez[2][2] = {
-                {sweep_march_tma_kernel<false, 0, T, 0, true, 5, 2>, sweep_march_tma_kernel<false, 1, T, 0, true, 5, 2>},
-                {sweep_march_tma_kernel<true, 0, T, 0, true, 5, 2>, sweep_march_tma_kernel<true, 1, T, 0, true, 5, 2>}};
-            kfn = ptablez[mp ? 1 : 0][kind1 ? 1 : 0];
-        }
-    } else if (ws == 1 || ws == 2) {
-        // mapped / Z weights of WENO5, FP64, face-independent coefficients
-        if constexpr (sizeof(T) == 8) {
-            static const KFn tablemz[2][2][2][2] = {
-                {{{sweep_march_tma_kernel<false, 0, T, 0, false, 5, 1>, sweep_march_tma_kernel<false, 0, T, 1, false, 5, 1>},
-                  {sweep_march_tma_kernel<false, 1, T, 0, false, 5, 1>, sweep_march_tma_kernel<false, 1, T, 1, false, 5, 1>}},
-                 {{sweep_march_tma_kernel<true, 0, T, 0, false, 5, 1>, sweep_march_tma_kernel<true, 0, T, 1, false, 5, 1>},
-                  {sweep_march_tma_kernel<true, 1, T, 0, false, 5, 1>, sweep_march_tma_kernel<true, 1, T, 1, false, 5, 1>}}},
-                {{{sweep_march_tma_kernel<false, 0, T, 0, false, 5, 2>, sweep_march_tma_kernel<false, 0, T, 1, false, 5, 2>},
-                  {sweep_march_tma_kernel<false, 1, T, 0, false, 5, 2>, sweep_march_tma_kernel<false, 1, T, 1, false, 5, 2>}},
-                 {{sweep_march_tma_kernel<true, 0, T, 0, false, 5, 2>, sweep_march_tma_kernel<true, 0, T, 1, false, 5, 2>},
-                  {sweep_march_tma_kernel<true, 1, T, 0, false, 5, 2>, sweep_march_tma_kernel<true, 1, T, 1, false, 5, 2>}}}};
-            kfn = tablemz[ws == 2 ? 1 : 0][mp ? 1 : 0][kind1 ? 1 : 0][ldr];
-        }
-    } else if (teno && a.ftab) {
-        // TENO with the per-face table (WENO5, WENO7): FP64 with TMA input tiles
-        if constexpr (sizeof(T) == 8) {
-            if (ldr) return 1003;
-            static const KFn ptablet[2][2][2] = {
-                {{sweep_march_tma_kernel<false, 0, T, 0, true, 5, 3>, sweep_march_tma_kernel<false, 1, T, 0, true, 5, 3>},
-                 {sweep_march_tma_kernel<true, 0, T, 0, true, 5, 3>, sweep_march_tma_kernel<true, 1, T, 0, true, 5, 3>}},
-                {{sweep_march_tma_kernel<false, 0, T, 0, true, 7, 3>, sweep_march_tma_kernel<false, 1, T, 0, true, 7, 3>},
-                 {sweep_march_tma_kernel<true, 0, T, 0, true, 7, 3>, sweep_march_tma_kernel<true, 1, T, 0, true, 7, 3>}}};
-            kfn = ptablet[order == 7 ? 1 : 0][mp ? 1 : 0][kind1 ? 1 : 0];
-        } else {
-            return 1003;
-        }
-    } else if (teno) {
-        // TENO weights, WENO5 or WENO7: face-independent coefficients
-        static const KFn tablet[2][2][2][2] = {
-            {{{sweep_march_tma_kernel<false, 0, T, 0, false, 5, 3>,
-               sweep_march_tma_kernel<false, 0, T, 1, false, 5, 3>},
-              {sweep_march_tma_kernel<false, 1, T, 0, false, 5, 3>,
-               sweep_march_tma_kernel<false, 1, T, 1, false, 5, 3>}},
-             {{sweep_march_tma_kernel<true, 0, T, 0, false, 5, 3>,
-               sweep_march_tma_kernel<true, 0, T, 1, false, 5, 3>},
-              {sweep_march_tma_kernel<true, 1, T, 0, false, 5, 3>,
-               sweep_march_tma_kernel<true, 1, T, 1, false, 5, 3>}}},
-            {{{sweep_march_tma_kernel<false, 0, T, 0, false, 7, 3>,
-               sweep_march_tma_kernel<false, 0, T, 1, false, 7, 3>},
-              {sweep_march_tma_kernel<false, 1, T, 0, false, 7, 3>,
-               sweep_march_tma_kernel<false, 1, T, 1, false, 7, 3>}},
-             {{sweep_march_tma_kernel<true, 0, T, 0, false, 7, 3>,
-               sweep_march_tma_kernel<true, 0, T, 1, false, 7, 3>},
-              {sweep_march_tma_kernel<true, 1, T, 0, false, 7, 3>,
-               sweep_march_tma_kernel<true, 1, T, 1, false, 7, 3>}}}};
-        kfn = tablet[order == 7 ? 1 : 0][mp ? 1 : 0][kind1 ? 1 : 0][ldr];
-    } else if (order == 3 && a.ftab) {
-        // WENO3-JS with the per-face table: FP64 with TMA input tiles
-        if constexpr (sizeof(T) == 8) {
-            if (ldr) return 1003;
-            static const KFn ptable3[2][2] = {
-                {sweep_march_tma_kernel<false, 0, T, 0, true, 3>, sweep_march_tma_kernel<false, 1, T, 0, true, 3>},
-                {sweep_march_tma_kernel<true, 0, T, 0, true, 3>, sweep_march_tma_kernel<true, 1, T, 0, true, 3>}};
-            kfn = ptable3[mp ? 1 : 0][kind1 ? 1 : 0];
-        } else {
-            return 1003;
-        }
-    } else if (order == 3) {
-        // WENO3: JS, face-independent coefficients
-        static const KFn table3[2][2][2] = {
-            {{sweep_march_tma_kernel<false, 0, T, 0, false, 3>, sweep_march_tma_kernel<false, 0, T, 1, false, 3>},
-             {sweep_march_tma_kernel<false, 1, T, 0, false, 3>, sweep_march_tma_kernel<false, 1, T, 1, false, 3>}},
-            {{sweep_march_tma_kernel<true, 0, T, 0, false, 3>, sweep_march_tma_kernel<true, 0, T, 1, false, 3>},
-             {sweep_march_tma_kernel<true, 1, T, 0, false, 3>, sweep_march_tma_kernel<true, 1, T, 1, false, 3>}}};
-        kfn = table3[mp ? 1 : 0][kind1 ? 1 : 0][ldr];
-    } else if (order == 7 && a.ftab) {
-        // WENO7-JS with the per-face table: FP64 with TMA input tiles
-        if constexpr (sizeof(T) == 8) {
-            if (ldr) return 1003;
-            static const KFn ptable7[2][2] = {
-                {sweep_march_tma_kernel<false, 0, T, 0, true, 7>, sweep_march_tma_kernel<false, 1, T, 0, true, 7>},
-                {sweep_march_tma_kernel<true, 0, T, 0, true, 7>, sweep_march_tma_kernel<true, 1, T, 0, true, 7>}};
-            kfn = ptable7[mp ? 1 : 0][kind1 ? 1 : 0];
-        } else {
-            return 1003;
-        }
-    } else if (order == 7) {
-        // WENO7: face-independent coefficients
-        static const KFn table7[2][2][2] = {
-            {{sweep_march_tma_kernel<false, 0, T, 0, false, 7>, sweep_march_tma_kernel<false, 0, T, 1, false, 7>},
-             {sweep_march_tma_kernel<false, 1, T, 0, false, 7>, sweep_march_tma_kernel<false, 1, T, 1, false, 7>}},
-            {{sweep_march_tma_kernel<true, 0, T, 0, false, 7>, sweep_march_tma_kernel<true, 0, T, 1, false, 7>},
-             {sweep_march_tma_kernel<true, 1, T, 0, false, 7>, sweep_march_tma_kernel<true, 1, T, 1, false, 7>}}};
-        kfn = table7[mp ? 1 : 0][kind1 ? 1 : 0][ldr];
-    } else if (a.ftab) {
-        // face-dependent coefficients: FP64 with TMA input tiles
-        if constexpr (sizeof(T) == 8) {
-            if (ldr) return 1003;
-            static const KFn ptable[2][2] = {
-                {sweep_march_tma_kernel<false, 0, T, 0, true>, sweep_march_tma_kernel<false, 1, T, 0, true>},
-                {sweep_march_tma_kernel<true, 0, T, 0, true>, sweep_march_tma_kernel<true, 1, T, 0, true>}};
-            kfn = ptable[mp ? 1 : 0][kind1 ? 1 : 0];
-        } else {
-            return 1003;
-        }
-    }
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kTmaWarps * 32, smem);
     if (occ < 1) return 1003;
+    march_segments(P.a, order, path == 2, 0, (long long)sms * occ * kTmaWarps);
     long long blocks = (a.n_items + kTmaWarps - 1) / kTmaWarps;
     const long long cap = (long long)sms * occ;
     if (blocks > cap) blocks = cap;

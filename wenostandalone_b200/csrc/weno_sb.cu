@@ -320,7 +320,7 @@ int launch_march_faces(const long long E[3], const SweepGeom& g, int dir, bool f
                        double* vL, double* vR, const CoefPtrs& cp, const WenoParams& wp, cudaStream_t st,
                        int ws = 0, int order = 5) {
     if (!cp.polyL || !cp.polyR || !cp.dL || !cp.dR || !cp.beta) return WENO_SB_ERR_UNSUPPORTED;
-    if (g.ns < 8 || ((uintptr_t)in & 15)) return WENO_SB_ERR_UNSUPPORTED;
+    if (g.ns < 8) return WENO_SB_ERR_UNSUPPORTED;
     const int rows = (int)g.ns + 16;
     double* tab = nullptr;
     // an error left by an earlier call is reported, not cleared by the
