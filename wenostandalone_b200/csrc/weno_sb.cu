@@ -6,6 +6,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -370,6 +371,13 @@ int run_weno(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsigned
     const bool mp = (flags & WENO_SB_F_MP) != 0;
     SweepGeom g = make_geom(d, dir, folded);
     if (g.nc < 1) return set_err(WENO_SB_ERR_ARG, "sweep has no core faces (Ns=%lld)", g.ns);
+    // v_rs_ws and the face states hold their columns back to back: one cross
+    // axis of all of them, so that only the sweep's last 32-column tile has
+    // idle lanes (212 columns per plane fill 7 tiles to 95%)
+    if (!folded && g.cols <= INT_MAX) {
+        g.c1 = g.cols;
+        g.c2 = g.nv = 1;
+    }
     CoefPtrs cp{nullptr, nullptr, nullptr, nullptr, nullptr};
     if (!ucf) cp = CoefPtrs{cf->polyL, cf->polyR, cf->dL, cf->dR, cf->beta_coef};
     WenoParams wp{gr->scheme, gr->weno_eps, gr->teno_CT};
