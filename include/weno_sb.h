@@ -186,8 +186,9 @@ int weno_sb_order1_dev(const weno_sb_grid *g, int dir, int dtype, const double *
                        void *vL, void *vR, void *stream);
 /* Reconstruction, order 3/5/7 (f90:392-1542).  v_in is v_rs_ws_dir, or
  * v_vf when flags has WENO_SB_F_FOLDED.  Per-face coefficient arrays take a
- * per-face table, allocated and freed stream-ordered on `stream`
- * (cudaMallocAsync). */
+ * per-face table, allocated and freed stream-ordered on `stream` (from a
+ * pool of the library that keeps at most 64 MB per device; within a stream
+ * capture, by the graph). */
 int weno_sb_weno_dev(const weno_sb_grid *g, int dir, int order, unsigned flags, int dtype,
                      const void *v_in, const weno_sb_coefs *coefs, void *vL, void *vR,
                      void *stream);

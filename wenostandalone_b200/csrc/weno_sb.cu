@@ -310,6 +310,67 @@ bool march_mapped_ok(const double* ucf) {
     return true;
 }
 
+// Id of the calling thread's current context, 0 when there is none or the
+// driver entry points are unavailable.
+unsigned long long current_context_id() {
+    typedef CUresult (*GetCurrentFn)(CUcontext*);
+    typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
+    static GetCurrentFn get_current = nullptr;
+    static GetIdFn get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = (GetCurrentFn)p;
+        p = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = (GetIdFn)p;
+    });
+    if (!get_current || !get_id) return 0;
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
+// Stream-ordered pool of the per-face tables.  The device's default pool
+// returns its memory at every synchronisation and maps it anew at the next
+// allocation (240-290 us measured for a 50 KB table, 3 us when kept); this
+// one keeps up to kTablePoolKeep bytes, two of the 32 MB pieces the driver
+// reserves at a time, and returns what is above that.  One per device and context (a cudaDeviceReset destroys it with its context);
+// null when the device has no pools.
+constexpr unsigned long long kTablePoolKeep = 64ull << 20;
+cudaMemPool_t table_pool() {
+    constexpr int kMaxDevices = 64;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    static unsigned long long ctxs[kMaxDevices] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    const unsigned long long ctx = current_context_id();
+    if (!pools[dev] || ctx == 0 || ctx != ctxs[dev]) {
+        pools[dev] = nullptr;
+        if (ctx == 0) return nullptr;  // contexts cannot be told apart
+        cudaMemPoolProps pr;
+        std::memset(&pr, 0, sizeof(pr));
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        unsigned long long keep = kTablePoolKeep;
+        if (cudaMemPoolCreate(&pools[dev], &pr) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            pools[dev] = nullptr;
+        }
+        ctxs[dev] = ctx;
+    }
+    return pools[dev];
+}
+
 // FP64 marching sweep with face-dependent coefficient arrays (WENO5 and
 // WENO7 with JS or TENO weights, WENO3-JS): the per-face table (one row per
 // face, 224 bytes for WENO5, 448 for WENO7, 96 for WENO3; ns + 16 rows: the kernel stages rows f0 .. f0 + 8
@@ -332,7 +393,13 @@ int launch_march_faces(const long long E[3], const SweepGeom& g, int dir, bool f
     // falls back to the one-thread-per-face kernels, which need no table;
     // during a stream capture the failed allocation has invalidated the
     // capture, so its error is returned instead
-    const cudaError_t ae = cudaMallocAsync((void**)&tab, sizeof(double) * pf_row_doubles(order) * (size_t)rows, st);
+    const size_t bytes = sizeof(double) * pf_row_doubles(order) * (size_t)rows;
+    // (in a capture the memory belongs to the graph, and no pool is made)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool direct = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    const cudaMemPool_t pool = direct ? table_pool() : nullptr;
+    const cudaError_t ae = pool ? cudaMallocFromPoolAsync((void**)&tab, bytes, pool, st)
+                                : cudaMallocAsync((void**)&tab, bytes, st);
     if (ae != cudaSuccess) {
         cudaGetLastError();
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1416,32 +1483,6 @@ static constexpr int kNoAllocMaxDevices = 64;
 static std::mutex g_noalloc_mu;
 static double* g_noalloc_addr[kNoAllocMaxDevices] = {};
 static unsigned long long g_noalloc_ctx[kNoAllocMaxDevices] = {};
-
-// Id of the calling thread's current context, 0 when there is none or the
-// driver entry points are unavailable.
-static unsigned long long current_context_id() {
-    typedef CUresult (*GetCurrentFn)(CUcontext*);
-    typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
-    static GetCurrentFn get_current = nullptr;
-    static GetIdFn get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = (GetCurrentFn)p;
-        p = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = (GetIdFn)p;
-    });
-    if (!get_current || !get_id) return 0;
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-    return id;
-}
 
 int weno_sb_checksum_noalloc(int dtype, const void* const* arrays, const int64_t* n, int count,
                              double* d_results, void* stream) {
