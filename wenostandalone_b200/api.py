@@ -13,6 +13,7 @@ device-pointer calls (arrays as 1-D CUDA tensors in Fortran element order).
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass
 
 import numpy as np
@@ -193,20 +194,38 @@ class Harness:
 # ---------------------------------------------------------------------------
 # Device-pointer API on CUDA tensors (1-D, Fortran element order)
 # ---------------------------------------------------------------------------
+# (A call's checks cost as much as its launch, 4.5 us, when written with
+# numpy products and torch's Stream objects: 26 us a call at 16^3 x 5 before,
+# and small blocks are bound by them.)
+_torch = None
+
+
+def _t():
+    """The torch module (imported at first use: the host-side functions of
+    this module need none)."""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
+
+
 def _ptr(t) -> int:
-    return 0 if t is None else int(t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _stream(stream) -> int:
     if stream is None:
-        import torch
+        torch = _t()
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None:
+            return raw(torch.cuda.current_device())
         return int(torch.cuda.current_stream().cuda_stream)
     return int(stream)
 
 
 def _dtype_of(t) -> int:
-    import torch
-    return L.FP32 if t.dtype == torch.float32 else L.FP64
+    return L.FP32 if t.dtype == _t().float32 else L.FP64
 
 
 def _need(name: str, t, n: int, dtypes) -> None:
@@ -214,7 +233,9 @@ def _need(name: str, t, n: int, dtypes) -> None:
     device-pointer entries take bare pointers, so the element type and count
     are checked here (a float32 array where FP64 is read, or a short array,
     would otherwise make the kernel access memory it does not own)."""
-    import torch
+    torch = _t()
+    if isinstance(t, torch.Tensor) and t.is_cuda and t.dtype in dtypes and t.is_contiguous() and t.numel() >= n:
+        return
     if t is None:
         raise ValueError(f"{name} is missing")
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
@@ -223,44 +244,60 @@ def _need(name: str, t, n: int, dtypes) -> None:
         raise TypeError(f"{name} has dtype {t.dtype}; expected {' or '.join(str(x) for x in dtypes)}")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    if t.numel() < n:
-        raise ValueError(f"{name} has {t.numel()} elements; the call accesses {n}")
+    raise ValueError(f"{name} has {t.numel()} elements; the call accesses {n}")
 
 
 def _f64():
-    import torch
-    return (torch.float64,)
+    return (_t().float64,)
+
+
+def _f64_32():
+    torch = _t()
+    return (torch.float64, torch.float32)
 
 
 def _same(t):
     return (t.dtype,) if t is not None else _f64()
 
 
+def _n_faces(grid: Grid) -> int:
+    """Elements of one face-state array (the same in every direction)."""
+    n1, n2, n3 = grid.N
+    return n1 * n2 * n3 * grid.v_size
+
+
+def _n_in(grid: Grid, d: int, folded: bool) -> int:
+    """Elements of a sweep's input: v_vf (folded) or v_rs_ws_d."""
+    if folded:
+        n1, n2, n3 = grid.N
+        return (n1 + 6) * (n2 + 6) * (n3 + 6) * grid.v_size
+    ns, c1, c2 = grid.extents(d)
+    return (ns + 6) * c1 * c2 * grid.v_size
+
+
 def _check_sweep(grid: Grid, d: int, v_in, vL, vR, folded: bool) -> None:
     """Sizes of a sweep's arrays; an invalid direction is left for the
     library to report (WENO_SB_ERR_ARG)."""
-    import torch
     if d not in (0, 1, 2):
         return
-    _need("vL", vL, int(np.prod(grid.face_shape(d))), (torch.float64, torch.float32))
-    _need("vR", vR, int(np.prod(grid.face_shape(d))), _same(vL))
-    n_in = int(np.prod(grid.vf_shape() if folded else grid.rs_shape(d)))
-    _need("v_in", v_in, n_in, _same(vL))
+    nf = _n_faces(grid)
+    _need("vL", vL, nf, _f64_32())
+    same = _same(vL)
+    _need("vR", vR, nf, same)
+    _need("v_in", v_in, _n_in(grid, d, folded), same)
 
 
 def reshape(grid: Grid, d: int, v_vf, out, stream=None) -> None:
-    import torch
-    _need("v_vf", v_vf, int(np.prod(grid.vf_shape())), _f64())
-    _need("out", out, int(np.prod(grid.rs_shape(d))), (torch.float64, torch.float32))
+    _need("v_vf", v_vf, _n_in(grid, d, True), _f64())
+    _need("out", out, _n_in(grid, d, False), _f64_32())
     check(lib().weno_sb_reshape_dev(ctypes.byref(grid.c()), d, _dtype_of(out), _ptr(v_vf), _ptr(out),
                                     _stream(stream)))
 
 
 def order1_copy(grid: Grid, d: int, v_vf, vL, vR, stream=None) -> None:
-    import torch
-    _need("v_vf", v_vf, int(np.prod(grid.vf_shape())), _f64())
-    _need("vL", vL, int(np.prod(grid.face_shape(d))), (torch.float64, torch.float32))
-    _need("vR", vR, int(np.prod(grid.face_shape(d))), _same(vL))
+    _need("v_vf", v_vf, _n_in(grid, d, True), _f64())
+    _need("vL", vL, math.prod(grid.face_shape(d)), _f64_32())
+    _need("vR", vR, math.prod(grid.face_shape(d)), _same(vL))
     check(lib().weno_sb_order1_dev(ctypes.byref(grid.c()), d, _dtype_of(vL), _ptr(v_vf), _ptr(vL), _ptr(vR),
                                    _stream(stream)))
 
@@ -318,11 +355,11 @@ def vjp(grid: Grid, d: int, order: int, v_in, coefs, gL, gR, gv, flags: int = 0,
         cs = coefs if isinstance(coefs, L.WenoCoefs) else coefs_struct(coefs)
         cs, fp = ctypes.byref(cs), None
     if d in (0, 1, 2) and order in (3, 5, 7):
-        n_in = int(np.prod(grid.vf_shape() if flags & L.F_FOLDED else grid.rs_shape(d)))
-        _need("v_in", v_in, n_in, _f64())
-        _need("gv", gv, n_in, _f64())
-        _need("gL", gL, int(np.prod(grid.face_shape(d))), _f64())
-        _need("gR", gR, int(np.prod(grid.face_shape(d))), _f64())
+        n_in, nf, f64 = _n_in(grid, d, bool(flags & L.F_FOLDED)), _n_faces(grid), _f64()
+        _need("v_in", v_in, n_in, f64)
+        _need("gv", gv, n_in, f64)
+        _need("gL", gL, nf, f64)
+        _need("gR", gR, nf, f64)
     check(lib().weno_sb_vjp_dev(ctypes.byref(grid.c()), d, order, flags, _ptr(v_in), cs, fp, _ptr(gL), _ptr(gR),
                                 _ptr(gv), _stream(stream)))
 
