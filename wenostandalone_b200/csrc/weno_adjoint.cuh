@@ -21,6 +21,9 @@
 // the kernel gathers them tile by tile through shared memory (no atomics).
 #pragma once
 
+#include <cmath>
+#include <type_traits>
+
 #include "weno_math.cuh"
 #include "sweep_generic.cuh"
 
@@ -397,6 +400,10 @@ __device__ void face_vjp(const double* v, const Coef<ORDER>& cf, int scheme, dou
 
 // ---------------------------------------------------------------------
 // Kernel: one thread per column (a, b, v) of the sweep, marching along it.
+// Columns may be cut into segments of cells (vjp_segments): a segment starts
+// 6 faces early, at the first face that reaches its cells.  (Blocks of four
+// warps: neighbouring columns share sectors, and with one-warp blocks WENO3
+// ran 12% slower at 128^3 x 5.)
 // Face o reads cells o..o+6 of the column (sweep index J = o + 3 + q,
 // q = -3..3) and contributes to the same cells; a cell has all its
 // contributions once face o = J is done.  The thread keeps the 7-cell
@@ -407,6 +414,7 @@ __device__ void face_vjp(const double* v, const Coef<ORDER>& cf, int scheme, dou
 // (coalesced); for sweeps along the contiguous axis the warp's 32 rows are
 // read through L1, each 32-byte sector serving four consecutive steps.
 // ---------------------------------------------------------------------
+constexpr int kVjpThreads = 128;
 struct VjpArgs {
     SweepGeom g;
     const double* v;
@@ -418,14 +426,24 @@ struct VjpArgs {
     WenoParams wp;
     int mp;
     int accumulate;
+    int seg, n_seg;  // cells per segment, segments per column
 };
 
 // UNI: face-independent coefficients, read from the kernel-parameter bank.
-template <int ORDER, bool UNI>
-__global__ void __launch_bounds__(128) vjp_kernel(const VjpArgs a) {
-    const long long ns = a.g.ns;
-    for (long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x; col < a.g.cols;
-         col += (long long)gridDim.x * blockDim.x) {
+// SEG: columns in segments; a kernel of its own, as the segment's bounds
+// cost whole columns 5-10% (WENO3: 1168 against 1057 us at 128^3 x 5).
+template <int ORDER, bool UNI, bool SEG>
+__global__ void __launch_bounds__(kVjpThreads, SEG && ORDER == 3 ? 3 : 0) vjp_kernel(const VjpArgs a) {
+    using Int = std::conditional_t<SEG, int, long long>;
+    const Int ns = (Int)a.g.ns;
+    const long long tiles = (a.g.cols + kVjpThreads - 1) / kVjpThreads;
+    for (long long item = SEG ? blockIdx.x : (long long)blockIdx.x * blockDim.x + threadIdx.x;
+         item < (SEG ? tiles * a.n_seg : a.g.cols); item += (long long)gridDim.x * (SEG ? 1 : blockDim.x)) {
+        const long long col = SEG ? item % tiles * kVjpThreads + threadIdx.x : item;
+        if (SEG && col >= a.g.cols) continue;
+        // cells [s0, s1), the last segment to the column's end
+        const Int s0 = SEG ? (Int)(item / tiles) * a.seg : 0, s1 = SEG ? min(s0 + a.seg, ns) : ns;
+        const Int o_begin = s0 > 6 ? s0 - 6 : 0;
         const long long av = col % a.g.c1;
         const long long tt = col / a.g.c1;
         const long long bv = tt % a.g.c2;
@@ -437,7 +455,7 @@ __global__ void __launch_bounds__(128) vjp_kernel(const VjpArgs a) {
         const long long sJ = a.g.sJ;
         double w[7], acc[7];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) w[q] = __ldg(vin + q * sJ);
+        for (int q = 0; q < 6; ++q) w[q] = __ldg(vin + (o_begin + q) * sJ);
 #pragma unroll
         for (int q = 0; q < 7; ++q) acc[q] = 0.0;
         // the new cell, the two cotangents and (accumulating) the old
@@ -447,27 +465,28 @@ __global__ void __launch_bounds__(128) vjp_kernel(const VjpArgs a) {
         // the gradient's read-modify-write among them, left the kernel
         // waiting on memory latency at every step).  Only this thread touches
         // the column's cells in this launch, so the old gradient read ahead
-        // is current.  Loads past the column's end read its last element and
+        // is current (outside a segment none is read: another warp
+        // may be writing those).  Loads past the column's end read its last element and
         // are not used.
-        const long long ncell = ns + 6;
+        const Int ncell = ns + 6;
         const bool acc_on = a.accumulate != 0;
-        auto fetch = [&](long long o, double& x, double& l, double& r, double& q) {
-            const long long jc = o + 6 < ncell ? o + 6 : ncell - 1;
-            const long long oc = o < ns ? o : ns - 1;
+        auto fetch = [&](Int o, double& x, double& l, double& r, double& q) {
+            const Int jc = o + 6 < ncell ? o + 6 : ncell - 1;
+            const Int oc = o < ns ? o : ns - 1;
             x = __ldg(vin + jc * sJ);
             l = __ldg(gLc + oc);
             r = __ldg(gRc + oc);
-            q = acc_on ? gout[oc * sJ] : 0.0;
+            q = acc_on && (!SEG || (oc >= s0 && oc < s1)) ? gout[oc * sJ] : 0.0;
         };
         constexpr int P = 4;
         double px[P], pl[P], pr[P], pq[P];
 #pragma unroll
-        for (int k = 0; k < P; ++k) fetch(k, px[k], pl[k], pr[k], pq[k]);
-        for (long long o0 = 0; o0 < ns; o0 += P) {
+        for (int k = 0; k < P; ++k) fetch(o_begin + k, px[k], pl[k], pr[k], pq[k]);
+        for (Int o0 = o_begin; o0 < s1; o0 += P) {
 #pragma unroll
             for (int k = 0; k < P; ++k) {
-                const long long o = o0 + k;
-                if (o >= ns) break;
+                const Int o = o0 + k;
+                if (o >= s1) break;
                 w[6] = px[k];
                 const double gLo = pl[k], gRo = pr[k], gvo = pq[k];
                 fetch(o + P, px[k], pl[k], pr[k], pq[k]);
@@ -486,7 +505,7 @@ __global__ void __launch_bounds__(128) vjp_kernel(const VjpArgs a) {
                     }
                 }
                 // cell J = o is complete
-                gout[o * sJ] = gvo + acc[0];
+                if (!SEG || o >= s0) gout[o * sJ] = gvo + acc[0];
 #pragma unroll
                 for (int q = 0; q < 6; ++q) {
                     acc[q] = acc[q + 1];
@@ -495,12 +514,32 @@ __global__ void __launch_bounds__(128) vjp_kernel(const VjpArgs a) {
                 acc[6] = 0.0;
             }
         }
+        if (SEG && s1 < ns) continue;
         // cells ns .. ns+5
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
             double* dst = gout + (ns + q) * sJ;
             if (a.accumulate) *dst += acc[q];
             else *dst = acc[q];
+        }
+    }
+}
+
+// Segments of a column for `ctas` resident CTAs: the cut for which they are
+// done first, as march_segments, with the 6 faces a segment starts early and
+// about 6 faces' time to fill its window.
+inline void vjp_segments(VjpArgs& a, long long ctas) {
+    const long long tiles = (a.g.cols + kVjpThreads - 1) / kVjpThreads;
+    double best = -1.0;
+    for (long long n = 1; n <= 16; ++n) {
+        const long long seg = (a.g.ns + n - 1) / n;
+        if (n > 1 && seg < 8) break;
+        const double exact = (double)(tiles * n) / (double)ctas;
+        const double cost = 0.5 * (exact + std::ceil(exact)) * (double)(seg + 6 + (n > 1 ? 6 : 0));
+        if (best < 0.0 || cost < best) {
+            best = cost;
+            a.seg = (int)seg;
+            a.n_seg = (int)((a.g.ns + seg - 1) / seg);
         }
     }
 }

@@ -555,20 +555,20 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
                                   num_sms());
         if (rc != WENO_SB_ERR_UNSUPPORTED) return rc == 0 ? cuda_err(cudaGetLastError(), "vjp march launch") : rc;
     }
-    const int threads = 128;
-    long long blocks = (a.g.cols + threads - 1) / threads;
-    if (blocks < 1) blocks = 1;
-    if (blocks > (1LL << 30)) blocks = 1LL << 30;
-    const unsigned grid = (unsigned)blocks;
-    switch (order * 2 + (uni ? 1 : 0)) {
-        case 6: vjp_kernel<3, false><<<grid, threads, 0, st>>>(a); break;
-        case 7: vjp_kernel<3, true><<<grid, threads, 0, st>>>(a); break;
-        case 10: vjp_kernel<5, false><<<grid, threads, 0, st>>>(a); break;
-        case 11: vjp_kernel<5, true><<<grid, threads, 0, st>>>(a); break;
-        case 14: vjp_kernel<7, false><<<grid, threads, 0, st>>>(a); break;
-        case 15: vjp_kernel<7, true><<<grid, threads, 0, st>>>(a); break;
-        default: return set_err(WENO_SB_ERR_ARG, "order must be 3, 5 or 7 (got %d)", order);
-    }
+    using KFn = void (*)(VjpArgs);
+    static const KFn table[3][2][2] = {
+        {{vjp_kernel<3, false, false>, vjp_kernel<3, false, true>}, {vjp_kernel<3, true, false>, vjp_kernel<3, true, true>}},
+        {{vjp_kernel<5, false, false>, vjp_kernel<5, false, true>}, {vjp_kernel<5, true, false>, vjp_kernel<5, true, true>}},
+        {{vjp_kernel<7, false, false>, vjp_kernel<7, false, true>}, {vjp_kernel<7, true, false>, vjp_kernel<7, true, true>}}};
+    if (order != 3 && order != 5 && order != 7)
+        return set_err(WENO_SB_ERR_ARG, "order must be 3, 5 or 7 (got %d)", order);
+    const KFn* const fn = table[(order - 3) / 2][uni ? 1 : 0];
+    int occ = 0;
+    WSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn[1], kVjpThreads, 0));
+    vjp_segments(a, (long long)num_sms() * std::max(occ, 1));
+    const KFn kfn = fn[a.n_seg > 1 ? 1 : 0];
+    const long long blocks = std::min<long long>((a.g.cols + kVjpThreads - 1) / kVjpThreads * a.n_seg, 1LL << 30);
+    kfn<<<(unsigned)blocks, kVjpThreads, 0, st>>>(a);
     return cuda_err(cudaGetLastError(), "vjp launch");
 }
 
