@@ -260,8 +260,6 @@ int launch_generic(const SweepGeom& g, int order, bool mp, const T* in, T* vL, T
     if (ucf)
         for (int q = 0; q < 56; ++q) uc.v[q] = ucf[q];
     switch (order * 2 + (mp ? 1 : 0)) {
-        case 0: launch_generic_t<0, false, T>(g, in, vL, vR, cp, wp, st, uc); break;
-        case 1: launch_generic_t<0, true, T>(g, in, vL, vR, cp, wp, st, uc); break;
         case 6: launch_generic_t<3, false, T>(g, in, vL, vR, cp, wp, st, uc); break;
         case 7: launch_generic_t<3, true, T>(g, in, vL, vR, cp, wp, st, uc); break;
         case 10: launch_generic_t<5, false, T>(g, in, vL, vR, cp, wp, st, uc); break;
@@ -271,6 +269,17 @@ int launch_generic(const SweepGeom& g, int order, bool mp, const T* in, T* vL, T
         default: return set_err(WENO_SB_ERR_ARG, "order must be 3, 5 or 7 (got %d)", order);
     }
     return cuda_err(cudaGetLastError(), "reconstruction launch");
+}
+
+// The standalone MP limiter on unfolded arrays.
+template <typename T>
+int launch_mp(const SweepGeom& g, const T* in, T* vL, T* vR, cudaStream_t st) {
+    if (g.nc < 1) return WENO_SB_OK;
+    constexpr long long per = (long long)kMpThreads * kMpFaces;
+    const long long blocks = (g.cols * g.nc + per - 1) / per;
+    mp_rows_kernel<T><<<(unsigned)std::min<long long>(blocks, (long long)num_sms() * 64), kMpThreads, 0, st>>>(
+        g.ns, g.cols, in, vL, vR);
+    return cuda_err(cudaGetLastError(), "MP limiter launch");
 }
 
 // Which implementation serves reconstruction sweeps, from WENO_SB_KERNEL
@@ -1323,12 +1332,9 @@ int weno_sb_preserve_monotonicity_dev(const weno_sb_grid* g, int dir, int dtype,
     if (rc || (rc = check_dir(dir)) || (rc = check_dtype(dtype))) return rc;
     if (!v_rs_ws || !vL || !vR) return set_err(WENO_SB_ERR_ARG, "NULL array pointer");
     SweepGeom sg = make_geom(d, dir, false);
-    CoefPtrs cp{nullptr, nullptr, nullptr, nullptr, nullptr};
-    WenoParams wp{g->scheme, g->weno_eps, g->teno_CT};
     cudaStream_t st = (cudaStream_t)stream;
-    if (dtype == WENO_SB_FP64)
-        return launch_generic<double>(sg, 0, true, (const double*)v_rs_ws, (double*)vL, (double*)vR, cp, wp, st);
-    return launch_generic<float>(sg, 0, true, (const float*)v_rs_ws, (float*)vL, (float*)vR, cp, wp, st);
+    if (dtype == WENO_SB_FP64) return launch_mp<double>(sg, (const double*)v_rs_ws, (double*)vL, (double*)vR, st);
+    return launch_mp<float>(sg, (const float*)v_rs_ws, (float*)vL, (float*)vR, st);
 }
 
 size_t weno_sb_checksum_scratch_bytes(int64_t n) {
