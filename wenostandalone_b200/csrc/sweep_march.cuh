@@ -128,27 +128,40 @@ struct BetaRow {
 // A face with a negative ideal weight gets a NaN in dL(0): its normalisation
 // test fails and the kernels redo it from the arrays, as the one-sided MP
 // median needs sign(v_L - v_0) = sign(E_L), which non-negative weights give.
-__global__ void march_face_table_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= rows) return;
-    auto core = [&](long long x) { x -= 3; return x < 0 ? 0 : (x > nc - 1 ? nc - 1 : x); };
-    const long long c = core(f);
-    double* row = tab + (long long)f * kFaceRow;
+// One thread per entry (all three table kernels): with one thread per row
+// they took 5 to 11 us a call, mostly the latency of its chained loads.
+__device__ __forceinline__ long long table_core(long long f, long long nc) {
+    f -= 3;
+    return f < 0 ? 0 : (f > nc - 1 ? nc - 1 : f);
+}
+// the ideal weights of core face c, R of them a side, hold a negative (or NaN)
+__device__ __forceinline__ bool table_negative(const CoefPtrs& cp, long long c, int R) {
     bool neg = false;
-    for (int r = 0; r < 3; ++r) {
-        const double dl = cp.dL[r + 5 * c], dr = cp.dR[r + 5 * c];
-        neg |= !(dl >= 0.0) || !(dr >= 0.0);
-        for (int s = 0; s < 2; ++s) {
-            row[2 * r + s] = dl * cp.polyL[c + nc * (r + 5 * s)];
-            row[6 + 2 * r + s] = dr * cp.polyR[c + nc * (r + 5 * s)];
-        }
-        row[12 + r] = dl;
-        row[15 + r] = dr;
-        const long long cr = core(f + r);
-        for (int s = 0; s < 3; ++s) row[18 + 3 * r + s] = cp.beta[cr + nc * (r + 5 * s)];
+    for (int r = 0; r < R; ++r) neg |= !(cp.dL[r + 5 * c] >= 0.0) || !(cp.dR[r + 5 * c] >= 0.0);
+    return neg;
+}
+__global__ void march_face_table_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long f = i / kFaceRow;
+    const int q = (int)(i % kFaceRow);
+    if (f >= rows) return;
+    const long long c = table_core(f, nc);
+    double x = 0.0;
+    if (q < 6) {
+        x = cp.dL[q / 2 + 5 * c] * cp.polyL[c + nc * (q / 2 + 5 * (q % 2))];
+    } else if (q < 12) {
+        const int k = q - 6;
+        x = cp.dR[k / 2 + 5 * c] * cp.polyR[c + nc * (k / 2 + 5 * (k % 2))];
+    } else if (q < 15) {
+        x = cp.dL[q - 12 + 5 * c];
+        if (q == 12 && table_negative(cp, c, 3)) x = __longlong_as_double(0x7ff8000000000000LL);
+    } else if (q < 18) {
+        x = cp.dR[q - 15 + 5 * c];
+    } else if (q < 27) {
+        const int r = (q - 18) / 3, t = (q - 18) % 3;
+        x = cp.beta[table_core(f + r, nc) + nc * (r + 5 * t)];
     }
-    if (neg) row[12] = __longlong_as_double(0x7ff8000000000000LL);
-    row[27] = 0.0;
+    tab[i] = x;
 }
 
 // Second-order minmod of the MP limiter (same decisions as mp_minmod /
@@ -850,27 +863,27 @@ struct Row7 {
 // kR7 likewise, dL, dR, and beta_coef(c(f + r), r, q).  A negative ideal
 // weight puts a NaN in dL(0), as march_face_table_kernel.
 __global__ void march_face_table7_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long f = i / kFaceRow7;
+    const int q = (int)(i % kFaceRow7);
     if (f >= rows) return;
-    auto core = [&](long long x) { x -= 3; return x < 0 ? 0 : (x > nc - 1 ? nc - 1 : x); };
-    const long long c = core(f);
-    double* row = tab + (long long)f * kFaceRow7;
-    bool neg = false;
-    for (int s = 0; s < 4; ++s) {
-        const double dl = cp.dL[s + 5 * c], dr = cp.dR[s + 5 * c];
-        neg |= !(dl >= 0.0) || !(dr >= 0.0);
-        for (int t = 0; t < 3; ++t) {
-            row[3 * s + t] = dl * cp.polyL[c + nc * ((3 - s) + 5 * t)];
-            row[12 + 3 * s + t] = dr * cp.polyR[c + nc * ((3 - s) + 5 * t)];
-        }
-        row[24 + s] = dl;
-        row[28 + s] = dr;
+    const long long c = table_core(f, nc);
+    double x;
+    if (q < 12) {
+        x = cp.dL[q / 3 + 5 * c] * cp.polyL[c + nc * (3 - q / 3 + 5 * (q % 3))];
+    } else if (q < 24) {
+        const int k = q - 12;
+        x = cp.dR[k / 3 + 5 * c] * cp.polyR[c + nc * (3 - k / 3 + 5 * (k % 3))];
+    } else if (q < 28) {
+        x = cp.dL[q - 24 + 5 * c];
+        if (q == 24 && table_negative(cp, c, 4)) x = __longlong_as_double(0x7ff8000000000000LL);
+    } else if (q < 32) {
+        x = cp.dR[q - 28 + 5 * c];
+    } else {
+        const int r = (q - 32) / 6, t = (q - 32) % 6;
+        x = cp.beta[table_core(f + r, nc) + nc * (r + 5 * t)];
     }
-    for (int r = 0; r < 4; ++r) {
-        const long long cr = core(f + r);
-        for (int q = 0; q < 6; ++q) row[32 + 6 * r + q] = cp.beta[cr + nc * (r + 5 * q)];
-    }
-    if (neg) row[24] = __longlong_as_double(0x7ff8000000000000LL);
+    tab[i] = x;
 }
 
 struct March64_7 {
@@ -1469,23 +1482,20 @@ struct Row3 {
 // dL(r) polyL(c, r, 0), kR likewise, dL, dR, beta_coef(c, r, 0).  A negative
 // ideal weight puts a NaN in dL(0).
 __global__ void march_face_table3_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long f = i / kFaceRow3;
+    const int q = (int)(i % kFaceRow3);
     if (f >= rows) return;
-    long long c = f - 3;
-    c = c < 0 ? 0 : (c > nc - 1 ? nc - 1 : c);
-    double* row = tab + (long long)f * kFaceRow3;
-    bool neg = false;
-    for (int r = 0; r < 2; ++r) {
-        const double dl = cp.dL[r + 5 * c], dr = cp.dR[r + 5 * c];
-        neg |= !(dl >= 0.0) || !(dr >= 0.0);
-        row[r] = dl * cp.polyL[c + nc * r];
-        row[2 + r] = dr * cp.polyR[c + nc * r];
-        row[4 + r] = dl;
-        row[6 + r] = dr;
-        row[8 + r] = cp.beta[c + nc * r];
-    }
-    row[10] = row[11] = 0.0;
-    if (neg) row[4] = __longlong_as_double(0x7ff8000000000000LL);
+    const long long c = table_core(f, nc);
+    double x = 0.0;
+    if (q < 2) x = cp.dL[q + 5 * c] * cp.polyL[c + nc * q];
+    else if (q < 4) x = cp.dR[q - 2 + 5 * c] * cp.polyR[c + nc * (q - 2)];
+    else if (q < 6) {
+        x = cp.dL[q - 4 + 5 * c];
+        if (q == 4 && table_negative(cp, c, 2)) x = __longlong_as_double(0x7ff8000000000000LL);
+    } else if (q < 8) x = cp.dR[q - 6 + 5 * c];
+    else if (q < 10) x = cp.beta[c + nc * (q - 8)];
+    tab[i] = x;
 }
 
 struct March64_3 {

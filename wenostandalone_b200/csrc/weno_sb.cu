@@ -416,9 +416,10 @@ int launch_march_faces(const long long E[3], const SweepGeom& g, int dir, bool f
             return cuda_err(ae, "per-face table allocation during stream capture");
         return WENO_SB_ERR_UNSUPPORTED;
     }
-    if (order == 7) march_face_table7_kernel<<<(rows + 127) / 128, 128, 0, st>>>(cp, g.nc, rows, tab);
-    else if (order == 3) march_face_table3_kernel<<<(rows + 127) / 128, 128, 0, st>>>(cp, g.nc, rows, tab);
-    else march_face_table_kernel<<<(rows + 127) / 128, 128, 0, st>>>(cp, g.nc, rows, tab);
+    const unsigned tb = (unsigned)(((long long)rows * pf_row_doubles(order) + 127) / 128);
+    if (order == 7) march_face_table7_kernel<<<tb, 128, 0, st>>>(cp, g.nc, rows, tab);
+    else if (order == 3) march_face_table3_kernel<<<tb, 128, 0, st>>>(cp, g.nc, rows, tab);
+    else march_face_table_kernel<<<tb, 128, 0, st>>>(cp, g.nc, rows, tab);
     MarchArgs a0 = make_march_args(g, in, vL, vR, wp, nullptr);
     a0.ftab = tab;
     a0.cp = cp;
