@@ -2,7 +2,7 @@
 // TENO weights and face-independent coefficients, marching along the sweep
 // like the forward kernel of sweep_march_tma.cuh.
 //
-// A warp owns 32 adjacent columns of one (w, v) and walks the whole column.
+// A warp owns 32 columns and walks a segment of their cells (vjp_march_cut).
 // At face J it recomputes the forward state from the carried window
 // (March64: the beta of the new difference pair, P_k, S_L, S_R, one
 // reciprocal) with the weights made explicit, then pulls the face's
@@ -31,6 +31,13 @@
 // [4 + 8k, 12 + 8k) of v, the cotangents of faces [4 + 8k, 12 + 8k) and
 // (accumulating) the old gradient of cells [4 + 8k, 12 + 8k), all completed
 // on one mbarrier.  Waits are bounded as in the forward kernel.
+//
+// LDR: arrays that TMA refuses (rows that are not 16-byte multiples, 8-byte
+// aligned bases) are staged by cp.async copies into the same tiles (eight
+// lanes per row where the rows run along the sweep), the tiles run over the
+// columns of all cross axes, and the gradient leaves by plain stores or
+// (accumulating) FP64 reductions, whose one add rounds as a load and an add
+// do.
 #pragma once
 
 #include <cuda.h>
@@ -52,9 +59,8 @@ struct VjpMarchArgs {
     int vbytes;         // one v (or old-gradient) tile
     int stage_bytes;    // v (and old gradient) tiles of one stage
     int warp_bytes;     // multiple of 1024
-    int ring_off;       // unused (0)
     unsigned tx_bytes;  // bytes one stage receives
-    const double* gLp;  // cotangents (ns, c1, c2, V), for the first core face
+    const double* gLp;  // cotangents (ns, c1, c2, V)
     const double* gRp;
 };
 
@@ -128,7 +134,7 @@ struct MarchVjp {
     // TENOW: TENO weights (f90:578-606), d_k delta_k / sum d delta with the
     // cutoff flags delta_k of the forward sequence; the flags are constant
     // between cutoff flips, so the weights pull nothing back to beta.
-    template <bool MPF, bool TENOW = false>
+    template <bool MPF, bool TENOW>
     __device__ __forceinline__ void face(const MarchArgs& a, double gLin, double gRin, int& pick, bool& ok) {
         const March64& w = f;
         ok = beta_ok(w.b0) && beta_ok(w.b1) && beta_ok(w.b2);
@@ -274,14 +280,15 @@ __device__ __forceinline__ void route_side(bool left, int code, double g, const 
     }
 }
 
-template <bool MPF, int KIND, bool TENOW = false>
+template <bool MPF, int KIND, bool TENOW, bool LDR>
 __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     vjp_march_kernel(const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tgL,
                      const __grid_constant__ CUtensorMap tgR, const __grid_constant__ CUtensorMap tgo,
                      const __grid_constant__ CUtensorMap tgs, const __grid_constant__ MarchArgs a,
                      const VjpMarchArgs t, double* __restrict__ gv) {
     constexpr int F = kTmaF, S = kVjpStages;
-    constexpr int XW = 34, XS = 1;  // column tiles: 34 cells from one left of column 0
+    // column tiles: 34 cells from one left of column 0 (TMA's 16-byte start)
+    constexpr int XW = LDR ? 32 : 34, XS = LDR ? 0 : 1;
     extern __shared__ __align__(1024) unsigned char smem_vj[];
     unsigned char* base = smem_vj + ((1024u - (smem_u32(smem_vj) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -289,11 +296,14 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     // per warp: the cotangent tiles of the S stages (gL, gR: 2048 bytes each,
     // 512-aligned for the swizzle), the field (and old-gradient) tiles of
     // the S stages, then one area that holds the per-lane corrections of a
-    // chunk and afterwards (row tiles) the outgoing [32 u][8 cells] tile
+    // chunk and afterwards (row tiles) the outgoing [32 u][8 cells] tile;
+    // LDR: the columns' offsets in the field and in the cotangents
     unsigned char* gring = wbase;
     unsigned char* vring = wbase + S * 4096;
     unsigned char* obuf = wbase + S * 4096 + S * t.stage_bytes;   // t.stage_bytes: v (+ old) per stage
     double* slot = (double*)obuf;  // 13 cells f0 .. f0+12 x 32 lanes
+    long long* offs = (long long*)(obuf + 13 * 32 * 8);
+    long long* offo = offs + 32;
     unsigned long long* bars = (unsigned long long*)(base + (size_t)kVjpWarps * t.warp_bytes) + warp * S;
     if (lane == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
@@ -306,15 +316,51 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     const long long ncell = a.ns + 6;
     unsigned n_issued = 0, n_waited = 0, n_out = 0;
     bool failed = false;
+    // this lane's column: its cells, its gradient, its cotangents' offset
+    const double* col = nullptr;
+    double* gcol = nullptr;
+    long long oo = 0;
 
     auto gstage = [&](unsigned k) { return gring + (size_t)(k % S) * 4096; };
     auto vstage = [&](unsigned k) { return vring + (size_t)(k % S) * t.stage_bytes; };
+    auto voff = [&](int p) -> unsigned {  // position p of this lane's column in a v / old-gradient tile
+        if constexpr (KIND == 0) return swz<double>((unsigned)lane, (unsigned)p);
+        else return (unsigned)((p * XW + lane + XS) * 8);
+    };
     auto issue = [&](unsigned k, int c, int u0, int w, int v) {
-        if (lane == 0) {
+        const int J0 = 4 + F * c;
+        unsigned char* sp = gstage(k);
+        unsigned char* vp = vstage(k);
+        if constexpr (LDR) {
+            // cells and faces past the column's end are zero-filled
+            auto copy8 = [&](const void* dst, const double* p, bool inb) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)), "l"(p),
+                             "r"(inb ? 8u : 0u)
+                             : "memory");
+            };
+            // rows along the sweep (the cotangents, and row tiles' cells):
+            // eight lanes per row, so one copy touches 4 rows, not 32
+            const int pp = lane & (F - 1), o = J0 + pp;
+#pragma unroll
+            for (int kk = 0; kk < F; ++kk) {
+                const int r = lane / F + (32 / F) * kk;
+                const unsigned so = swz<double>((unsigned)r, (unsigned)pp);
+                const long long co = offo[r] + (o < ns ? o : 0);
+                copy8(sp + so, t.gLp + co, o < ns);
+                copy8(sp + 2048 + so, t.gRp + co, o < ns);
+                if constexpr (KIND == 0)
+                    copy8(vp + so, (const double*)a.in + offs[r] + (o < ncell ? o : 0), o < ncell);
+            }
+            if constexpr (KIND == 1) {
+#pragma unroll
+                for (int p = 0; p < F; ++p) {
+                    const bool in = J0 + p < ncell;
+                    copy8(vp + voff(p), col + (in ? J0 + p : 0) * a.sJ, in);
+                }
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        } else if (lane == 0) {
             unsigned long long* bar = &bars[k % S];
-            unsigned char* sp = gstage(k);
-            unsigned char* vp = vstage(k);
-            const int J0 = 4 + F * c;
             const int cU = t.uoff + u0, cW = t.woff + w;
             mbar_arrive_expect_tx(bar, t.tx_bytes);
             const int o1 = t.odimU == 1 ? u0 : w, o2 = t.odimU == 2 ? u0 : w;
@@ -328,62 +374,107 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
         }
     };
     auto wait_stage = [&](unsigned k) -> bool {
-        if (!mbar_wait(&bars[k % S], (k / S) & 1u)) return false;
+        if constexpr (LDR) {
+            // copy groups issued after stage k may stay in flight
+            const unsigned after = n_issued - (k + 1);
+            if (after >= 2) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+            else if (after == 1) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncwarp();  // the rows are filled by eight lanes each
+        } else {
+            if (!mbar_wait(&bars[k % S], (k / S) & 1u)) return false;
+        }
         n_waited = k + 1;
         return true;
     };
-    auto voff = [&](int p) -> unsigned {  // position p of this lane's column in a v / old-gradient tile
-        if constexpr (KIND == 0) return swz<double>((unsigned)lane, (unsigned)p);
-        else return (unsigned)((p * XW + lane + XS) * 8);
-    };
     auto cell = [&](unsigned k, int p) -> double { return *(const double*)(vstage(k) + voff(p)); };
     auto oldg = [&](unsigned k, int p) -> double {
-        return t.acc ? *(const double*)(vstage(k) + t.vbytes + voff(p)) : 0.0;
+        if constexpr (LDR) return 0.0;  // added by the reductions
+        else return t.acc ? *(const double*)(vstage(k) + t.vbytes + voff(p)) : 0.0;
     };
     auto cot = [&](unsigned k, int arr, int i) -> double {
         return *(const double*)(gstage(k) + arr * 2048 + swz<double>((unsigned)lane, (unsigned)i));
     };
+    // generic pull-back of face o on the cells c7 = J-3 .. J+3
+    auto redo = [&](const double* c7, double gL, double gR, double* acc7) {
+        Coef<5> cf;
+        for (int q = 0; q < 6; ++q) { cf.pL[q] = a.ucf[q]; cf.pR[q] = a.ucf[6 + q]; }
+        for (int q = 0; q < 3; ++q) { cf.dL[q] = a.ucf[12 + q]; cf.dR[q] = a.ucf[15 + q]; }
+        for (int q = 0; q < 9; ++q) cf.b[q] = a.ucf[18 + q];
+        face_vjp<5>(c7 + 3, cf, TENOW ? TENO : JS, a.wp.eps, a.wp.teno_ct, MPF, gL, gR, acc7);
+    };
 
     for (long long item = (long long)blockIdx.x * kVjpWarps + warp; item < a.n_items && !failed; item += nwarps) {
-        long long tt = item;
-        const int ut = (int)(tt % a.n_ut);
-        tt /= a.n_ut;
-        const int wv = (int)(tt % a.Nw);
-        const int vv = (int)(tt / a.Nw);
-        const int u0 = ut * 32;
-        const bool live = u0 + lane < a.Nu;
-        const int uc = live ? u0 + lane : a.Nu - 1;
-        const double* col = (const double*)a.in + a.in_off + uc * a.sU + wv * a.sW + vv * a.sV;
-        double* gcol = gv + a.in_off + uc * a.sU + wv * a.sW + vv * a.sV;
-        const int nch = (ns + 1) / F + 1;       // chunks until cell ns+5 is out
+        const int sg = (int)(item % a.n_seg);
+        long long tt = item / a.n_seg;
+        int u0 = 0, wv = 0, vv = 0, c_end = 32;
+        bool live;
+        long long u, wl, vl;
+        if constexpr (LDR) {
+            const long long c0 = tt * 32;
+            live = c0 + lane < a.n_cols;
+            c_end = a.n_cols - c0 < 32 ? (int)(a.n_cols - c0) : 32;
+            tt = live ? c0 + lane : a.n_cols - 1;  // idle lanes shadow the last column
+            u = tt % a.Nu;
+            tt /= a.Nu;
+            wl = tt % a.Nw;
+            vl = tt / a.Nw;
+        } else {
+            u0 = (int)(tt % a.n_ut) * 32;
+            tt /= a.n_ut;
+            wv = (int)(tt % a.Nw);
+            vv = (int)(tt / a.Nw);
+            live = u0 + lane < a.Nu;
+            u = live ? u0 + lane : a.Nu - 1;
+            wl = wv;
+            vl = vv;
+        }
+        {
+            const long long io = a.in_off + u * a.sU + wl * a.sW + vl * a.sV;
+            col = (const double*)a.in + io;
+            gcol = gv + io;
+            oo = u * a.oU + wl * a.oW + vl * a.oV;
+            // (the previous item's readers of the offsets synced since)
+            if constexpr (LDR) {
+                offs[lane] = io;
+                offo[lane] = oo;
+                __syncwarp();
+            }
+        }
+        // chunks [cs, ce) are written; a segment starts one chunk early, whose
+        // faces reach its first cells
+        const int n_all = (ns + 1) / F + 1;     // chunks until cell ns+5 is out
+        const int cs = sg * a.seg, ce = cs + a.seg < n_all ? cs + a.seg : n_all;
+        const int cb = cs > 0 ? cs - 1 : 0;
+        const int nch = ce - cb;
         const int ntiles = nch + 1;
         const unsigned k0 = n_issued;
-        for (int k = 0; k < ntiles && k < S; ++k) issue(k0 + k, k, u0, wv, vv);
-        n_issued += (ntiles < S ? ntiles : S);
+        for (int k = 0; k < ntiles && k < S; ++k) {
+            issue(k0 + k, cb + k, u0, wv, vv);
+            ++n_issued;
+        }
         if (!wait_stage(k0)) { failed = true; break; }
 
-        // cells 0..3 receive nothing; face 3 (cells 4..8 = stage 0 positions
-        // 0..4) starts the window
-        if (live && !t.acc)
+        // the window of the face before the first chunk, f0 - 1 (cells
+        // f0 .. f0+4 = positions 0..4 of the first stage)
+        // cells 0..3 receive nothing
+        if (live && !t.acc && sg == 0)
             for (int q = 0; q < 4; ++q) gcol[q * a.sJ] = 0.0;
         MarchVjp m;
         m.init(a, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
-        {
-            const long long oi = 3 + (long long)uc * a.oU + wv * a.oW + vv * a.oV;
-            const double gL = live ? __ldg(t.gLp + oi) : 0.0, gR = live ? __ldg(t.gRp + oi) : 0.0;
+        if (cb == 0) {
+            // face 3 (a later segment's reaches only cells of the
+            // chunk it does not write)
+            const double gL = live ? __ldg(t.gLp + oo + 3) : 0.0, gR = live ? __ldg(t.gRp + oo + 3) : 0.0;
             int pk;
             bool ok;
-            m.face<MPF, TENOW>(a, gL, gR, pk, ok);
+            m.template face<MPF, TENOW>(a, gL, gR, pk, ok);
             if (pk || (!ok && live)) {
                 // cells 3..9 of the column = J-3 .. J+3 of face 3 (J = 6)
                 double c7[7], acc7[7] = {0, 0, 0, 0, 0, 0, 0};
                 for (int q = 0; q < 7; ++q) c7[q] = __ldg(col + (3 + q) * a.sJ);
                 if (!ok) {
-                    Coef<5> cf;
-                    for (int q = 0; q < 6; ++q) { cf.pL[q] = a.ucf[q]; cf.pR[q] = a.ucf[6 + q]; }
-                    for (int q = 0; q < 3; ++q) { cf.dL[q] = a.ucf[12 + q]; cf.dR[q] = a.ucf[15 + q]; }
-                    for (int q = 0; q < 9; ++q) cf.b[q] = a.ucf[18 + q];
-                    face_vjp<5>(c7 + 3, cf, JS, a.wp.eps, 0.0, MPF, gL, gR, acc7);
+                    redo(c7, gL, gR, acc7);
                 } else {
                     route_side(true, pk & 7, gL, c7 + 1, acc7 + 1);
                     route_side(false, pk >> 3, gR, c7 + 1, acc7 + 1);
@@ -396,16 +487,17 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 m.gcp1 += acc7[4] + acc7[5];
                 m.gdp1 += acc7[5];
             }
-            (void)m.advance(a, cell(k0, 5));  // cell 3: nothing
         }
-        // chunk c: faces f0 .. f0+7 (f0 = 4 + 8c); face f0+i pushes cell
+        (void)m.advance(a, cell(k0, 5));  // cell f0 - 1: not written here
+        // chunk c: faces f0 .. f0+7 (f0 = 4 + 8 (cb + c)); face f0+i pushes cell
         // f0+i+6 = stage c position 6+i (i < 2) or stage c+1 position i-2,
         // and emits cell f0+i = position i of stage c's tiles
         for (int c = 0; c < nch; ++c) {
             const unsigned kc = k0 + c;
             if (!wait_stage(kc + 1)) { failed = true; break; }
-            const int f0 = 4 + F * c;
-            if constexpr (KIND == 0) {
+            const int f0 = 4 + F * (cb + c);
+            const bool emit = cb + c >= cs;
+            if constexpr (KIND == 0 && !LDR) {
                 if (n_out >= 1) {
                     if (lane == 0) bulk_wait_read0();
                     __syncwarp();
@@ -422,7 +514,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 const double gR = valid ? cot(kc, 1, i) : 0.0;
                 int pk;
                 bool ok;
-                m.face<MPF, TENOW>(a, gL, gR, pk, ok);
+                m.template face<MPF, TENOW>(a, gL, gR, pk, ok);
                 picks |= (unsigned long long)(valid ? pk : 0) << (6 * i);
                 bad |= (ok || !valid) ? 0u : (1u << i);
                 outv[i] = m.advance(a, (i < 2) ? cell(kc, 6 + i) : cell(kc + 1, i - 2)) + oldg(kc, i);
@@ -436,8 +528,8 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 for (int k = 0; k < 13; ++k) slot[k * 32 + lane] = 0.0;
                 for (int i = 0; i < F; ++i) {
                     const int pk = (int)((picks >> (6 * i)) & 63ull);
-                    const bool redo = (bad >> i) & 1u;
-                    if (!pk && !redo) continue;
+                    const bool again = (bad >> i) & 1u;
+                    if (!pk && !again) continue;
                     // cells f0+i .. f0+i+6 = J-3 .. J+3 (J = f0+i+3)
                     double c7[7], acc7[7] = {0, 0, 0, 0, 0, 0, 0};
                     for (int q = 0; q < 7; ++q) {
@@ -445,12 +537,8 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                         c7[q] = k < 8 ? cell(kc, k) : cell(kc + 1, k - 8);
                     }
                     const double gL = cot(kc, 0, i), gR = cot(kc, 1, i);
-                    if (redo) {
-                        Coef<5> cf;
-                        for (int q = 0; q < 6; ++q) { cf.pL[q] = a.ucf[q]; cf.pR[q] = a.ucf[6 + q]; }
-                        for (int q = 0; q < 3; ++q) { cf.dL[q] = a.ucf[12 + q]; cf.dR[q] = a.ucf[15 + q]; }
-                        for (int q = 0; q < 9; ++q) cf.b[q] = a.ucf[18 + q];
-                        face_vjp<5>(c7 + 3, cf, TENOW ? TENO : JS, a.wp.eps, a.wp.teno_ct, MPF, gL, gR, acc7);
+                    if (again) {
+                        redo(c7, gL, gR, acc7);
                     } else {
                         route_side(true, pk & 7, gL, c7 + 1, acc7 + 1);
                         route_side(false, pk >> 3, gR, c7 + 1, acc7 + 1);
@@ -467,32 +555,54 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 m.gcm1 += slot[10 * 32 + lane];
                 m.gc0 += slot[11 * 32 + lane];
                 m.gcp1 += slot[12 * 32 + lane];
+                // (every lane's slots are read before the outgoing tile, which
+                // shares their memory, is written)
+                if constexpr (KIND == 0) __syncwarp();
             }
-            if constexpr (KIND == 0) {
-                unsigned char* ob = obuf;
+            if (emit) {
+                if constexpr (KIND == 0) {
+                    unsigned char* ob = obuf;
 #pragma unroll
-                for (int i = 0; i < F; ++i) *(double*)(ob + swz<double>((unsigned)lane, (unsigned)i)) = outv[i];
-                fence_async_shared();
-                __syncwarp();
-                if (lane == 0) {
-                    const int cU = t.uoff + u0, cW = t.woff + wv;
-                    const int c0 = t.dimJ == 0 ? f0 : (t.dimU == 0 ? cU : cW);
-                    const int c1 = t.dimJ == 1 ? f0 : (t.dimU == 1 ? cU : cW);
-                    const int c2 = t.dimJ == 2 ? f0 : (t.dimU == 2 ? cU : cW);
-                    tma_store_4d(&tgs, ob, c0, c1, c2, vv);
-                    bulk_commit();
-                }
-                ++n_out;
-            } else {
+                    for (int i = 0; i < F; ++i) *(double*)(ob + swz<double>((unsigned)lane, (unsigned)i)) = outv[i];
+                    if constexpr (LDR) {
+                        __syncwarp();
+                        const int fi = lane & (F - 1);
+                        if (f0 + fi < ncell) {
+#pragma unroll 4
+                            for (int cc = lane / F; cc < c_end; cc += 32 / F) {
+                                double* g = gv + offs[cc] + f0 + fi;
+                                const double x = *(const double*)(ob + swz<double>((unsigned)cc, (unsigned)fi));
+                                if (t.acc) atomicAdd(g, x);
+                                else *g = x;
+                            }
+                        }
+                    } else {
+                        fence_async_shared();
+                        __syncwarp();
+                        if (lane == 0) {
+                            const int cU = t.uoff + u0, cW = t.woff + wv;
+                            const int c0 = t.dimJ == 0 ? f0 : (t.dimU == 0 ? cU : cW);
+                            const int c1 = t.dimJ == 1 ? f0 : (t.dimU == 1 ? cU : cW);
+                            const int c2 = t.dimJ == 2 ? f0 : (t.dimU == 2 ? cU : cW);
+                            tma_store_4d(&tgs, ob, c0, c1, c2, vv);
+                            bulk_commit();
+                        }
+                        ++n_out;
+                    }
+                } else {
 #pragma unroll
-                for (int i = 0; i < F; ++i) {
-                    const long long J = (long long)f0 + i;
-                    if (live && J < ncell) gcol[J * a.sJ] = outv[i];
+                    for (int i = 0; i < F; ++i) {
+                        const long long J = (long long)f0 + i;
+                        if (live && J < ncell) {
+                            if (LDR && t.acc) atomicAdd(gcol + J * a.sJ, outv[i]);
+                            else gcol[J * a.sJ] = outv[i];
+                        }
+                    }
                 }
             }
             __syncwarp();
             if (c + S < ntiles) {
-                issue(kc + S, c + S, u0, wv, vv);
+                issue(kc + S, cb + c + S, u0, wv, vv);
                 ++n_issued;
             }
         }
@@ -501,25 +611,47 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     if (failed) {
         for (unsigned k = n_waited; k < n_issued; ++k) mbar_wait(&bars[k % S], (k / S) & 1u);
     }
-    if (lane == 0) bulk_wait_all();
+    if (LDR) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    else if (lane == 0) bulk_wait_all();
     __syncwarp();
 }
 
-// Host side: the marching adjoint for FP64 WENO5-JS with face-independent
-// coefficients.  Returns 1003 (unsupported) when a tensor map cannot be
-// made (16-byte alignment of bases and strides, an even face count); the
-// caller then runs vjp_kernel.  gv must already hold what is to be added to
-// when acc is set.
+// Cut the columns' chunks into segments for `warps` resident warps, as
+// march_segments: a segment runs one chunk more than it writes, and takes
+// about a chunk's time to start.
+inline void vjp_march_cut(MarchArgs& a, long long tiles, long long warps) {
+    const long long chunks = (a.ns + 1) / kTmaF + 1;
+    double best = -1.0;
+    for (long long n = 1; n <= chunks; ++n) {
+        const long long c = (chunks + n - 1) / n;
+        if (n > 1 && c == (chunks + n - 2) / (n - 1)) continue;
+        const long long nseg = (chunks + c - 1) / c;
+        const double exact = (double)(tiles * nseg) / (double)warps;
+        const double cost = 0.5 * (exact + std::ceil(exact)) * (double)(c + 1 + (nseg > 1 ? 1 : 0));
+        if (best < 0.0 || cost < best) {
+            best = cost;
+            a.seg = (int)c;
+            a.n_seg = (int)nseg;
+        }
+    }
+    a.n_items = tiles * a.n_seg;
+}
+
+// Host side: the marching adjoint for FP64 WENO5 with JS or TENO weights and
+// face-independent coefficients.  TMA staging when every base and row is a
+// 16-byte multiple, copies by the lanes otherwise.  Returns 1003 (unsupported) for sweeps of fewer than
+// 8 faces or a lane axis the march arguments did not choose; the caller then
+// runs vjp_kernel.  gv must already hold what is to be added to when acc is
+// set.
 inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, bool acc,
                             const double* v, const double* ucf, const WenoParams& wp, const double* gL,
                             const double* gR, double* gv, cudaStream_t st, int sms) {
     EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) return 1003;
-    if ((((uintptr_t)v) | ((uintptr_t)gL) | ((uintptr_t)gR) | ((uintptr_t)gv)) & 15) return 1003;
-    if (g.ns < 8 || (g.ns & 1) || g.nc < 1) return 1003;
+    if (g.ns < 8 || g.nc < 1) return 1003;
     MarchArgs a = make_march_args(g, v, nullptr, nullptr, wp, ucf);
     VjpMarchArgs t{};
     const bool kind1 = folded && dir != 0;
+    if (kind1 != (a.sU == 1)) return 1003;
     t.kind = kind1 ? 1 : 0;
     t.acc = acc ? 1 : 0;
     t.gLp = gL;
@@ -549,58 +681,55 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
     strides[0] = dims[0] * 8;
     strides[1] = dims[0] * dims[1] * 8;
     strides[2] = dims[0] * dims[1] * dims[2] * 8;
-    if (strides[0] % 16) return 1003;
-    if ((t.kind == 1) != (a.sU == 1)) return 1003;
     const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
     CUtensorMap mv, mL, mR, mo, ms;
-    std::memset(&mo, 0, sizeof(mo));
-    std::memset(&ms, 0, sizeof(ms));
+    for (CUtensorMap* m : {&mv, &mL, &mR, &mo, &ms}) std::memset(m, 0, sizeof(*m));
     auto make = [&](CUtensorMap* m, const void* p, const cuuint64_t* d, const cuuint64_t* s2, const cuuint32_t* b,
                     CUtensorMapSwizzle z) {
         return enc(m, dt, 4, (void*)p, d, s2, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, z,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
-    if (!make(&mv, v, dims, strides, box, swz)) return 1003;
-    if (acc && !make(&mo, gv, dims, strides, box, swz)) return 1003;
-    if (!kind1) {
-        // the store map ends at the last column of the sweep, so the lanes
-        // past it (the last 32-column tile) write nothing
-        cuuint64_t sd[4] = {dims[0], dims[1], dims[2], dims[3]};
-        sd[t.dimU] = (cuuint64_t)(t.uoff + a.Nu);
-        if (!make(&ms, gv, sd, strides, box, swz)) return 1003;
-    }
     cuuint64_t od[4] = {(cuuint64_t)g.ns, (cuuint64_t)g.c1, (cuuint64_t)g.c2, (cuuint64_t)g.nv};
     cuuint64_t os[3] = {(cuuint64_t)g.ns * 8, (cuuint64_t)(g.ns * g.c1) * 8, (cuuint64_t)(g.ns * g.c1 * g.c2) * 8};
     cuuint32_t ob[4] = {kTmaF, 1, 1, 1};
     t.odimU = (a.oU == g.ns) ? 1 : 2;
     ob[t.odimU] = 32;
-    if (!make(&mL, gL, od, os, ob, CU_TENSOR_MAP_SWIZZLE_64B) || !make(&mR, gR, od, os, ob, CU_TENSOR_MAP_SWIZZLE_64B))
-        return 1003;
-    // one item per 32-column tile of a whole column
-    a.seg = (int)g.ns;
-    a.n_seg = 1;
-    a.n_items = (long long)a.n_ut * a.Nw * a.NV;
-    t.stage_bytes = t.vbytes * (acc ? 2 : 1);   // field (+ old gradient) tiles of one stage
-    t.ring_off = 0;
-    t.warp_bytes = ((kVjpStages * 4096 + kVjpStages * t.stage_bytes + 13 * 32 * 8 + 1023) / 1024) * 1024;
-    t.tx_bytes = (unsigned)(2 * 2048 + t.vbytes * (acc ? 2 : 1));
+    // the store map (row tiles) ends at the last column of the sweep, so the
+    // lanes past it (the last 32-column tile) write nothing
+    cuuint64_t sd[4] = {dims[0], dims[1], dims[2], dims[3]};
+    sd[t.dimU] = (cuuint64_t)(t.uoff + a.Nu);
+    const bool tma = enc && ((((uintptr_t)v) | ((uintptr_t)gL) | ((uintptr_t)gR) | ((uintptr_t)gv)) & 15) == 0 &&
+                     (g.ns & 1) == 0 && strides[0] % 16 == 0 && make(&mv, v, dims, strides, box, swz) &&
+                     (!acc || make(&mo, gv, dims, strides, box, swz)) &&
+                     (kind1 || make(&ms, gv, sd, strides, box, swz)) &&
+                     make(&mL, gL, od, os, ob, CU_TENSOR_MAP_SWIZZLE_64B) &&
+                     make(&mR, gR, od, os, ob, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (tma) {
+        t.stage_bytes = t.vbytes * (acc ? 2 : 1);   // field (+ old gradient) tiles of one stage
+        t.tx_bytes = (unsigned)(2 * 2048 + t.vbytes * (acc ? 2 : 1));
+    } else {
+        t.stage_bytes = 2048;
+    }
+    t.warp_bytes = kVjpStages * (4096 + t.stage_bytes) + 13 * 32 * 8;
+    if (!tma) t.warp_bytes += 2 * 32 * 8;
+    t.warp_bytes = (t.warp_bytes + 511) / 512 * 512;
     const size_t smem = 1024 + (size_t)kVjpWarps * t.warp_bytes + (size_t)kVjpWarps * kVjpStages * 8;
     using KFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, VjpMarchArgs,
                          double*);
-    const bool teno = wp.scheme == TENO;
-    static const KFn table[2][2][2] = {
-        {{vjp_march_kernel<false, 0, false>, vjp_march_kernel<false, 1, false>},
-         {vjp_march_kernel<true, 0, false>, vjp_march_kernel<true, 1, false>}},
-        {{vjp_march_kernel<false, 0, true>, vjp_march_kernel<false, 1, true>},
-         {vjp_march_kernel<true, 0, true>, vjp_march_kernel<true, 1, true>}}};
-    const KFn kfn = table[teno ? 1 : 0][mp ? 1 : 0][kind1 ? 1 : 0];
+#define WSB_VJP_ROW(MPF, TENOW)                                                      \
+    {{vjp_march_kernel<MPF, 0, TENOW, false>, vjp_march_kernel<MPF, 1, TENOW, false>}, \
+     {vjp_march_kernel<MPF, 0, TENOW, true>, vjp_march_kernel<MPF, 1, TENOW, true>}}
+    static const KFn table[2][2][2][2] = {{WSB_VJP_ROW(false, false), WSB_VJP_ROW(true, false)},
+                                          {WSB_VJP_ROW(false, true), WSB_VJP_ROW(true, true)}};
+#undef WSB_VJP_ROW
+    const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][tma ? 0 : 1][kind1 ? 1 : 0];
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kVjpWarps * 32, smem);
     if (occ < 1) return 1003;
-    long long blocks = (a.n_items + kVjpWarps - 1) / kVjpWarps;
     const long long cap = (long long)sms * occ;
-    if (blocks > cap) blocks = cap;
+    vjp_march_cut(a, tma ? (long long)a.n_ut * a.Nw * a.NV : (a.n_cols + 31) / 32, cap * kVjpWarps);
+    const long long blocks = std::min((a.n_items + kVjpWarps - 1) / kVjpWarps, cap);
     kfn<<<(unsigned)blocks, kVjpWarps * 32, smem, st>>>(mv, mL, mR, mo, ms, a, t, gv);
     return 0;
 }

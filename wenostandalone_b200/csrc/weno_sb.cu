@@ -380,6 +380,30 @@ cudaMemPool_t table_pool() {
     return pools[dev];
 }
 
+// A table of n doubles on `st`, for the caller to cudaFreeAsync.  Returns
+// WENO_SB_ERR_UNSUPPORTED when no stream-ordered allocation (or no memory)
+// is available: the caller falls back to the kernels that need no table.
+int table_alloc(double** tab, size_t n, cudaStream_t st) {
+    // an error left by an earlier call is reported, not cleared by the
+    // allocation's own error handling below
+    const cudaError_t pending = cudaPeekAtLastError();
+    if (pending != cudaSuccess) return cuda_err(cudaGetLastError(), "error pending before the per-face table");
+    // (in a capture the memory belongs to the graph, and no pool is made)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool direct = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    const cudaMemPool_t pool = direct ? table_pool() : nullptr;
+    const cudaError_t ae = pool ? cudaMallocFromPoolAsync((void**)tab, sizeof(double) * n, pool, st)
+                                : cudaMallocAsync((void**)tab, sizeof(double) * n, st);
+    if (ae == cudaSuccess) return WENO_SB_OK;
+    cudaGetLastError();
+    // during a stream capture the failed allocation has invalidated the
+    // capture, so its error is returned instead
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+        return cuda_err(ae, "per-face table allocation during stream capture");
+    return WENO_SB_ERR_UNSUPPORTED;
+}
+
 // FP64 marching sweep with face-dependent coefficient arrays (WENO5 and
 // WENO7 with JS or TENO weights, WENO3-JS): the per-face table (one row per
 // face, 224 bytes for WENO5, 448 for WENO7, 96 for WENO3; ns + 16 rows: the kernel stages rows f0 .. f0 + 8
@@ -394,28 +418,8 @@ int launch_march_faces(const long long E[3], const SweepGeom& g, int dir, bool f
     if (g.ns < 8) return WENO_SB_ERR_UNSUPPORTED;
     const int rows = (int)g.ns + 16;
     double* tab = nullptr;
-    // an error left by an earlier call is reported, not cleared by the
-    // allocation's own error handling below
-    const cudaError_t pending = cudaPeekAtLastError();
-    if (pending != cudaSuccess) return cuda_err(cudaGetLastError(), "error pending before the per-face table");
-    // no stream-ordered allocation available (or no memory): the caller
-    // falls back to the one-thread-per-face kernels, which need no table;
-    // during a stream capture the failed allocation has invalidated the
-    // capture, so its error is returned instead
-    const size_t bytes = sizeof(double) * pf_row_doubles(order) * (size_t)rows;
-    // (in a capture the memory belongs to the graph, and no pool is made)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool direct = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-    const cudaMemPool_t pool = direct ? table_pool() : nullptr;
-    const cudaError_t ae = pool ? cudaMallocFromPoolAsync((void**)&tab, bytes, pool, st)
-                                : cudaMallocAsync((void**)&tab, bytes, st);
-    if (ae != cudaSuccess) {
-        cudaGetLastError();
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
-            return cuda_err(ae, "per-face table allocation during stream capture");
-        return WENO_SB_ERR_UNSUPPORTED;
-    }
+    const int arc = table_alloc(&tab, (size_t)rows * pf_row_doubles(order), st);
+    if (arc) return arc;
     const unsigned tb = (unsigned)(((long long)rows * pf_row_doubles(order) + 127) / 128);
     if (order == 7) march_face_table7_kernel<<<tb, 128, 0, st>>>(cp, g.nc, rows, tab);
     else if (order == 3) march_face_table3_kernel<<<tb, 128, 0, st>>>(cp, g.nc, rows, tab);
