@@ -79,7 +79,11 @@ constexpr int kPfOut = WSB_MTMA_PF_OUTBUF;
 constexpr int kPstStages = 3;
 constexpr int kPstOut = 2;
 __host__ __device__ constexpr int mtma_stages(bool pf, bool pst) { return pst ? kPstStages : (pf ? kPfStages : kTmaStages); }
-__host__ __device__ constexpr int mtma_outs(bool pf, bool pst) { return pst ? kPstOut : (pf ? kPfOut : kTmaOut); }
+// (FP64 WENO3 has the registers for four CTAs per SM, and the shared memory
+// with one output tile: 1353 against 1389 us at 200^3 x 8)
+__host__ __device__ constexpr int mtma_outs(bool pf, bool pst, int order, int es) {
+    return pst ? kPstOut : (pf ? kPfOut : (order == 3 && es == 8 ? 1 : kTmaOut));
+}
 // rows f0 .. f0 + 8 of a chunk (WENO5 / WENO7 table rows)
 __host__ __device__ constexpr int pf_row_doubles(int order) {
     return order == 7 ? kFaceRow7 : (order == 3 ? kFaceRow3 : kFaceRow);
@@ -183,6 +187,7 @@ struct MtmaGeo {
     void* vR;
     long long ns, sJ, sU, sW, sV, in_off, oU, oW, oV;
     int Nu, Nw, n_ut, seg, n_seg, pad_;
+    long long n_cols;
 };
 struct MtmaItemArgs {
     MtmaGeo geo;
@@ -203,7 +208,7 @@ inline MtmaGeo mtma_geo(const MarchArgs& a) {
     g.in = a.in; g.vL = a.vL; g.vR = a.vR;
     g.ns = a.ns; g.sJ = a.sJ; g.sU = a.sU; g.sW = a.sW; g.sV = a.sV; g.in_off = a.in_off;
     g.oU = a.oU; g.oW = a.oW; g.oV = a.oV;
-    g.Nu = a.Nu; g.Nw = a.Nw; g.n_ut = a.n_ut; g.seg = a.seg; g.n_seg = a.n_seg;
+    g.Nu = a.Nu; g.Nw = a.Nw; g.n_ut = a.n_ut; g.seg = a.seg; g.n_seg = a.n_seg; g.n_cols = a.n_cols;
     return g;
 }
 struct MtmaEntry {
@@ -227,13 +232,11 @@ __device__ __forceinline__ const auto& mtma_geo_of(const MarchArgs& a, const Mtm
 // (face_mapped; FP64 WENO5, face-independent coefficients), 2 Z (face_z;
 // FP64 WENO5), 3 TENO (face_teno).  MULTI: the work items of
 // several sweeps (entries ents[0 .. n_ents), items numbered entry after
-// entry); each item finds its entry, whose geometry, maps, loader (TMA or
-// per lane) and store kind (TMA or plain) it uses, with the coefficients of
-// the kernel's MarchArgs.
-// PST (single sweeps): per-lane loads and plain stores, compiled in.  A lane
-// may then hold any column, so the tiles run over the columns of all cross
-// axes in turn (u fastest, then w, v) and only the sweep's last tile has
-// idle lanes.
+// entry); each item finds its entry, whose geometry and maps it uses, with
+// the coefficients of the kernel's MarchArgs.
+// PST: per-lane loads and plain stores.  A lane may then hold any column, so
+// the tiles run over the columns of all cross axes in turn (u fastest, then
+// w, v) and only the sweep's last tile has idle lanes.
 template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER, int WS, bool MULTI, bool PST = false>
 __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CUtensorMap* toutL0,
                                                const CUtensorMap* toutR0, const MarchArgs& a, const MarchTmaArgs& t,
@@ -244,7 +247,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                   "mapped / Z weights: the FP64 WENO5 engine");
     static_assert(WS != 1 || !PF, "mapped weights: face-independent coefficients");
     constexpr int F = kTmaF, S = mtma_stages(PF, PST);
-    constexpr int NOUT = mtma_outs(PF, PST);                // output tiles per warp
+    constexpr int NOUT = mtma_outs(PF, PST, ORDER, (int)sizeof(T));  // output tiles per warp
     constexpr unsigned OB = 32u * F * sizeof(T);          // one output array tile
     constexpr int XW = sizeof(T) == 8 ? 34 : 36;          // KIND 1 tile width
     constexpr int XS = sizeof(T) == 8 ? 1 : 3;            // KIND 1 column of lane 0
@@ -268,10 +271,12 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     unsigned char* obuf = wbase;
     unsigned char* ring = wbase + t.ring_off;
     unsigned long long* bars = (unsigned long long*)(base + (size_t)kTmaWarps * warp_bytes) + warp * S;
-    // after the mbarriers: the warp's argument slot (grouped sweeps), or its
+    // after the mbarriers: the warp's argument slot (grouped sweeps) and its
     // columns' offsets in the face arrays (PST)
-    MtmaSlot* slot = (MtmaSlot*)(base + (size_t)kTmaWarps * warp_bytes + (size_t)kTmaWarps * S * 8 +
-                                 (size_t)warp * kMtmaSlot);
+    unsigned char* extra = base + (size_t)kTmaWarps * warp_bytes + (size_t)kTmaWarps * S * 8 +
+                           (size_t)warp * (MULTI && PST ? 2 : 1) * kMtmaSlot;
+    MtmaSlot* slot = (MtmaSlot*)extra;
+    long long* offs = (long long*)(extra + (MULTI ? kMtmaSlot : 0));
     if (lane == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -281,20 +286,10 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     const long long nwarps = (long long)gridDim.x * kTmaWarps;
     unsigned n_issued = 0, n_waited = 0;      // tiles requested / completed (waited on) by this warp
     unsigned n_chunks = 0;                    // output chunks stored by this warp
-    // grouped sweeps mix tiles loaded by TMA (completed on the stage's
-    // mbarrier) with tiles copied per lane (no mbarrier phase): bit s is the
-    // parity of the next phase of stage s's mbarrier
-    unsigned ph = 0;
     bool failed = false;
 
     auto tile_ptr = [&](unsigned k) { return ring + (size_t)(k % S) * t.stage_bytes; };
-    auto parity = [&](unsigned k) -> unsigned {
-        if constexpr (MULTI) return (ph >> (k % S)) & 1u;
-        else return (k / S) & 1u;
-    };
-    auto phase_done = [&](unsigned k) {
-        if constexpr (MULTI) ph ^= 1u << (k % S);
-    };
+    auto parity = [&](unsigned k) -> unsigned { return (k / S) & 1u; };
     // per-face table rows (PF): in global memory, and the chunk's rows
     // staged with input tile k
     auto row = [&](int f) { return a.ftab + (long long)f * RW; };
@@ -330,8 +325,8 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             if (lane < NW)
                 reinterpret_cast<unsigned long long*>(&slot->ia)[lane] =
                     __ldg(reinterpret_cast<const unsigned long long*>(&E->ia) + lane);
-            if (lane == 0) {
-                slot->e = E;
+            if (lane == 0) slot->e = E;
+            if (!PST && lane == 0) {
                 // the entry's maps are read by the TMA unit from global
                 // memory, where a table freed and allocated again may hold
                 // other maps at the same address: drop any copy cached for
@@ -354,11 +349,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         auto mapI = [&]() { return MULTI ? &slot->e->tin : tin0; };
         auto mapL = [&]() { return MULTI ? &slot->e->toutL : toutL0; };
         auto mapR = [&]() { return MULTI ? &slot->e->toutR : toutR0; };
-        const bool ldr = MULTI ? te.ldr != 0 : LDR == 1;
-        // plain stores (face rows not 16-byte multiples): per entry in grouped
-        // sweeps, a kernel of its own for a single sweep (as a branch beside
-        // the TMA stores it cost the face body two registers and a spill)
-        const bool pst = MULTI ? te.pst != 0 : PST;
+        constexpr bool ldr = LDR == 1;
         T* __restrict__ outL = (T*)g.vL;
         T* __restrict__ outR = (T*)g.vR;
         // faces written: the core faces 3 .. ns-4 (chunks from face 4, face 3 by
@@ -453,7 +444,6 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         auto wait_tile = [&](unsigned k) -> bool {
             if (!ldr) {
                 if (!mbar_wait(&bars[k % S], parity(k))) return false;
-                phase_done(k);
             } else {
                 // copy groups issued after tile k may stay in flight (every
                 // tile of earlier items has been waited on)
@@ -475,12 +465,11 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         long long tt = li / g.n_seg;
         int u0 = 0, wv = 0, vv = 0;
         int c_end = 32;            // PST: columns of this tile
-        long long* offs = (long long*)slot;
         if constexpr (PST) {
             const long long c0 = tt * 32;
-            live = c0 + lane < a.n_cols;
-            c_end = a.n_cols - c0 < 32 ? (int)(a.n_cols - c0) : 32;
-            tt = live ? c0 + lane : a.n_cols - 1;  // idle lanes shadow the last column
+            live = c0 + lane < g.n_cols;
+            c_end = g.n_cols - c0 < 32 ? (int)(g.n_cols - c0) : 32;
+            tt = live ? c0 + lane : g.n_cols - 1;  // idle lanes shadow the last column
             const long long u = tt % g.Nu;
             tt /= g.Nu;
             const long long w = tt % g.Nw, v = tt / g.Nw;
@@ -501,11 +490,6 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         const int nch = f_end > f_start ? (f_end - f_start + F - 1) / F : 0;
         const int ntiles = nch + 1;                               // tiles 0 .. nch
         const unsigned k0 = n_issued;                             // first tile of this item
-        if (MULTI && !ldr) {
-            // the ring's stages may last have been written by per-lane copies
-            fence_async_shared();
-            __syncwarp();
-        }
         for (int k = 0; k < ntiles && k < S; ++k) issue(k0 + k, f_start + F * k, u0, wv, vv);
         n_issued += (ntiles < S ? ntiles : S);
         if (!wait_tile(k0)) { failed = true; break; }
@@ -586,15 +570,10 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             // the store issued from this buffer NOUT chunks ago must have read
             // it before the chunk's face states are written: waited here, or
             // (one output buffer) just before the first write, so the first
-            // faces' arithmetic overlaps it.  A chunk of plain stores waits
-            // for every store in flight (grouped sweeps: the last bulk store
-            // may be the one from this buffer)
+            // faces' arithmetic overlaps it
             const bool wait_out = !PST && n_chunks >= (unsigned)NOUT;
             if (NOUT > 1 && wait_out) {
-                if (lane == 0) {
-                    if (MULTI && pst) bulk_wait_read0();
-                    else bulk_wait_read1();
-                }
+                if (lane == 0) bulk_wait_read1();
                 __syncwarp();
             }
             unsigned bad = 0;
@@ -730,24 +709,6 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                         }
                     }
                 }
-            } else if (pst) {
-                // plain stores: lane l writes face f0 + l % 8 of columns
-                // l / 8, l / 8 + 4, ..., so one instruction writes four
-                // columns' runs of 8 consecutive faces
-                __syncwarp();
-                const int fi = lane & (F - 1);
-                if (fi < nF) {
-                    // (a rolled loop with one running index: unrolled, its
-                    // addresses took 24 registers of the face body)
-                    const int u_end = g.Nu - u0 < 32 ? g.Nu - u0 : 32;
-                    const long long step = (long long)(32 / F) * g.oU;
-                    long long oi = (long long)(f0 + fi) + (long long)(u0 + lane / F) * g.oU + wv * g.oW + vv * g.oV;
-#pragma unroll 1
-                    for (int cc = lane / F; cc < u_end; cc += 32 / F, oi += step) {
-                        outL[oi] = *(const T*)(ob + swz<T>((unsigned)cc, (unsigned)fi));
-                        outR[oi] = *(const T*)(ob + OB + swz<T>((unsigned)cc, (unsigned)fi));
-                    }
-                }
             } else {
                 const int i_last = ORDER == 3 ? -1 : o_last - 1 - f0;  // the last core face, when in this chunk
                 if (i_last >= 0 && i_last < F && live) {
@@ -782,10 +743,9 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         // (only TMA tiles fail, and an item's tiles are all of one kind)
         for (unsigned k = n_waited; k < n_issued; ++k) {
             mbar_wait(&bars[k % S], parity(k));
-            phase_done(k);
         }
     }
-    if (LDR == 1 || MULTI) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (LDR == 1) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     if (lane == 0) bulk_wait_all();
     __syncwarp();
 }
@@ -796,13 +756,17 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
 #ifndef WSB_MTMA_MIN_BLOCKS_W7
 #define WSB_MTMA_MIN_BLOCKS_W7 2  // WENO7 carries ~27 doubles of state: 3 CTAs per SM would spill
 #endif
-#define WSB_MTMA_BOUNDS(ORDER, T)                                                      \
-    __launch_bounds__(kTmaWarps * 32, (ORDER) == 7 ? WSB_MTMA_MIN_BLOCKS_W7            \
-                                                   : (sizeof(T) == 8 ? WSB_MTMA_MIN_BLOCKS : WSB_MTMA_MIN_BLOCKS_F32))
+// CTAs per SM by order (WENO3: 4, but 3 with plain stores, whose second
+// output tile leaves no shared memory for a fourth)
+template <int ORDER, typename T, bool PST>
+constexpr int kMtmaMinBlocks = ORDER == 7 ? WSB_MTMA_MIN_BLOCKS_W7
+                               : ORDER == 3 && !(PST && sizeof(T) == 8)
+                                   ? 4
+                                   : (sizeof(T) == 8 ? WSB_MTMA_MIN_BLOCKS : WSB_MTMA_MIN_BLOCKS_F32);
 
 // One sweep: maps and arguments in the parameter bank.
 template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER = 5, int WS = 0, bool PST = false>
-__global__ void WSB_MTMA_BOUNDS(ORDER, T)
+__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST>))
     sweep_march_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap toutL,
                            const __grid_constant__ CUtensorMap toutR, const __grid_constant__ MarchArgs a,
                            const MarchTmaArgs t) {
@@ -812,27 +776,17 @@ __global__ void WSB_MTMA_BOUNDS(ORDER, T)
 
 // A group of sweeps in one launch: entries (64-byte aligned, in global
 // memory, written before the launch) in item order, n_items in all;
-// coefficients and shared-memory layout of the group in a and t.
-// CTAs per SM the FP64 grouped kernels are bounded for: column tiles 3
-// (WENO5's body fits 168 registers there), row tiles 2 (at 3 their WENO5
-// body spills 36-44 bytes and runs 2-3% slower); FP32 3.
-#ifndef WSB_MTMA_MULTI_MIN_BLOCKS
-#define WSB_MTMA_MULTI_MIN_BLOCKS 2     // FP64 row tiles
-#endif
-#ifndef WSB_MTMA_MULTI_MIN_BLOCKS_K1
-#define WSB_MTMA_MULTI_MIN_BLOCKS_K1 3  // FP64 column tiles
-#endif
-template <bool MPF, int KIND, typename T, int ORDER, int WS>
-__global__ void __launch_bounds__(kTmaWarps * 32,
-                                  ORDER == 7 ? WSB_MTMA_MIN_BLOCKS_W7
-                                             : (sizeof(T) == 8 ? (KIND == 1 ? WSB_MTMA_MULTI_MIN_BLOCKS_K1
-                                                                            : WSB_MTMA_MULTI_MIN_BLOCKS)
-                                                               : WSB_MTMA_MIN_BLOCKS_F32))
+// coefficients and shared-memory layout of the group in a and t.  PST: a
+// group of sweeps whose layouts TMA refuses (a kernel of its own: with both
+// loaders and both stores in one body, chosen per entry, the row-tile body
+// ran at two CTAs per SM).
+template <bool MPF, int KIND, typename T, int ORDER, int WS, bool PST>
+__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST>))
     sweep_march_tma_multi_kernel(const MtmaEntry* __restrict__ ents, const long long* __restrict__ item0s,
                                  int n_ents, long long n_items, const __grid_constant__ MarchArgs a,
                                  const MarchTmaArgs t) {
-    march_tma_body<MPF, KIND, T, 0, false, ORDER, WS, true>(nullptr, nullptr, nullptr, a, t, ents, item0s, n_ents,
-                                                              n_items);
+    march_tma_body<MPF, KIND, T, PST ? 1 : 0, false, ORDER, WS, true, PST>(nullptr, nullptr, nullptr, a, t, ents, item0s,
+                                                                           n_ents, n_items);
 }
 
 // Host side.  A sweep's plan: its maps, arguments and shared-memory layout.
@@ -893,7 +847,7 @@ void march_layout(MtmaPlan& P, int order, bool pst) {
     MarchTmaArgs& t = P.t;
     const bool pf = P.a.ftab != nullptr;
     const int nst = mtma_stages(pf, pst);
-    const int out_bytes = mtma_outs(pf, pst) * 2 * 32 * kTmaF * (int)sizeof(T);
+    const int out_bytes = mtma_outs(pf, pst, order, (int)sizeof(T)) * 2 * 32 * kTmaF * (int)sizeof(T);
     t.ring_off = out_bytes;
     t.rows_off = out_bytes + nst * t.stage_bytes;
     t.warp_bytes = ((t.rows_off + (pf ? nst * pf_chunk_bytes(order) : 0) + 1023) / 1024) * 1024;
@@ -985,8 +939,10 @@ int plan_march_tma(const long long E[3], const SweepGeom& g, int dir, bool folde
         t.pst = 0;
     // the lane axis must be the one the march arguments chose
     if ((t.kind == 1) != (a.sU == 1)) return 1003;
-    march_segments(a, order, false, seg_faces, (long long)sms * kTmaWarps * 3);
-    march_layout<T>(P, order, false);
+    // (a single sweep's launch cuts and lays out anew for its kernel)
+    const bool plain = t.ldr || t.pst;
+    march_segments(a, order, plain, seg_faces, (long long)sms * kTmaWarps * 3);
+    march_layout<T>(P, order, plain);
     return 0;
 }
 
@@ -1055,7 +1011,7 @@ int launch_march_tma(const long long E[3], const SweepGeom& g, int dir, bool fol
     const int path = t.pst || (pf && t.ldr) ? 2 : t.ldr;
     const MtmaFn kfn = mtma_kernel<T>(order, ws, pf, mp, t.kind == 1, path);
     if (!kfn) return 1003;
-    if (path == 2) march_layout<T>(P, order, true);
+    march_layout<T>(P, order, path == 2);
     const size_t smem = P.smem;
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int occ = 0;
@@ -1069,21 +1025,26 @@ int launch_march_tma(const long long E[3], const SweepGeom& g, int dir, bool fol
     return 0;
 }
 
-// Kernel of a group of sweeps, by storage T, order, weights, MP and tile
-// kind (null for WENO3 with TENO weights, which no engine covers).
+// Kernel of a group of sweeps, by storage T, order, weights, MP, tile kind
+// and plain stores (null for WENO3 with TENO weights, which no engine covers).
 using MtmaMultiFn = void (*)(const MtmaEntry*, const long long*, int, long long, MarchArgs, MarchTmaArgs);
-template <typename T, int ORDER, int WS>
+template <typename T, int ORDER, int WS, bool PST>
 MtmaMultiFn mtma_multi_pick(bool mp, bool kind1) {
-    static const MtmaMultiFn tab[2][2] = {
-        {sweep_march_tma_multi_kernel<false, 0, T, ORDER, WS>, sweep_march_tma_multi_kernel<false, 1, T, ORDER, WS>},
-        {sweep_march_tma_multi_kernel<true, 0, T, ORDER, WS>, sweep_march_tma_multi_kernel<true, 1, T, ORDER, WS>}};
+    static const MtmaMultiFn tab[2][2] = {{sweep_march_tma_multi_kernel<false, 0, T, ORDER, WS, PST>,
+                                           sweep_march_tma_multi_kernel<false, 1, T, ORDER, WS, PST>},
+                                          {sweep_march_tma_multi_kernel<true, 0, T, ORDER, WS, PST>,
+                                           sweep_march_tma_multi_kernel<true, 1, T, ORDER, WS, PST>}};
     return tab[mp ? 1 : 0][kind1 ? 1 : 0];
 }
-template <typename T>
+template <typename T, bool PST>
 MtmaMultiFn mtma_multi_kernel(int order, bool teno, bool mp, bool kind1) {
-    if (order == 3) return teno ? nullptr : mtma_multi_pick<T, 3, 0>(mp, kind1);
-    if (order == 7) return teno ? mtma_multi_pick<T, 7, 3>(mp, kind1) : mtma_multi_pick<T, 7, 0>(mp, kind1);
-    return teno ? mtma_multi_pick<T, 5, 3>(mp, kind1) : mtma_multi_pick<T, 5, 0>(mp, kind1);
+    if (order == 3) return teno ? nullptr : mtma_multi_pick<T, 3, 0, PST>(mp, kind1);
+    if (order == 7) return teno ? mtma_multi_pick<T, 7, 3, PST>(mp, kind1) : mtma_multi_pick<T, 7, 0, PST>(mp, kind1);
+    return teno ? mtma_multi_pick<T, 5, 3, PST>(mp, kind1) : mtma_multi_pick<T, 5, 0, PST>(mp, kind1);
+}
+template <typename T>
+MtmaMultiFn mtma_multi_kernel(int order, bool teno, bool mp, bool kind1, bool plain) {
+    return plain ? mtma_multi_kernel<T, true>(order, teno, mp, kind1) : mtma_multi_kernel<T, false>(order, teno, mp, kind1);
 }
 
 }  // namespace wsb

@@ -611,6 +611,7 @@ constexpr int kBatchMaxBranches = 16;
 // Mode 2: the sweeps of one grouped launch.
 struct MtmaGroup {
     int fp32 = 0, order = 5, teno = 0, mp = 0, kind = 0;
+    bool plain = false;       // layouts TMA refuses: per-lane loads and plain stores
     MarchArgs a{};            // coefficients of the group (its first entry's arguments)
     MarchTmaArgs t{};         // shared-memory layout (the same for every entry)
     size_t smem = 0;
@@ -793,10 +794,11 @@ int batch_plan_groups(Batch* B, int seg_faces) {
                                                     (double*)e.vR, a0, num_sms(), e.order, seg_faces, P);
                 const bool teno = e.wp.scheme == WENO_SB_TENO;
                 if (prc == 0 && !(e.order == 3 && teno)) {
+                    const bool plain = P.t.ldr || P.t.pst;
                     MtmaGroup* G = nullptr;
                     for (auto& q : B->groups)
                         if (q.fp32 == e.fp32 && q.order == e.order && q.teno == (int)teno && q.mp == e.mp &&
-                            q.kind == P.t.kind && march_coefs_equal(q.a, P.a)) {
+                            q.kind == P.t.kind && q.plain == plain && march_coefs_equal(q.a, P.a)) {
                             G = &q;
                             break;
                         }
@@ -808,6 +810,7 @@ int batch_plan_groups(Batch* B, int seg_faces) {
                         G->teno = teno ? 1 : 0;
                         G->mp = e.mp;
                         G->kind = P.t.kind;
+                        G->plain = plain;
                         G->a = P.a;
                         G->t = P.t;
                         // plus the warps' argument slots
@@ -862,8 +865,9 @@ int batch_enqueue_groups(Batch* B, cudaStream_t st) {
         load[k] += u.first;
         if (u.second >= 0) {
             const MtmaGroup& G = B->groups[(size_t)u.second];
-            const MtmaMultiFn kfn = G.fp32 ? mtma_multi_kernel<float>(G.order, G.teno != 0, G.mp != 0, G.kind == 1)
-                                           : mtma_multi_kernel<double>(G.order, G.teno != 0, G.mp != 0, G.kind == 1);
+            const MtmaMultiFn kfn = G.fp32 ? mtma_multi_kernel<float>(G.order, G.teno != 0, G.mp != 0, G.kind == 1, G.plain)
+                                           : mtma_multi_kernel<double>(G.order, G.teno != 0, G.mp != 0, G.kind == 1,
+                                                                       G.plain);
             if (!kfn) { rc = set_err(WENO_SB_ERR_UNSUPPORTED, "no grouped kernel for a batch group"); break; }
             rc = cuda_err(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.smem),
                           "cudaFuncSetAttribute");
