@@ -349,35 +349,39 @@ unsigned long long current_context_id() {
 // returns its memory at every synchronisation and maps it anew at the next
 // allocation (240-290 us measured for a 50 KB table, 3 us when kept); this
 // one keeps up to kTablePoolKeep bytes, two of the 32 MB pieces the driver
-// reserves at a time, and returns what is above that.  One per device and context (a cudaDeviceReset destroys it with its context);
-// null when the device has no pools.
+// reserves at a time, and returns what is above that.  One per device and
+// context (a cudaDeviceReset destroys it with its context); null when the
+// device has no pools or contexts cannot be told apart.
 constexpr unsigned long long kTablePoolKeep = 64ull << 20;
 cudaMemPool_t table_pool() {
-    constexpr int kMaxDevices = 64;
+    struct Pool {
+        int dev;
+        unsigned long long ctx;
+        cudaMemPool_t pool;
+    };
     static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    static unsigned long long ctxs[kMaxDevices] = {};
+    static std::vector<Pool> pools;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lk(mu);
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     const unsigned long long ctx = current_context_id();
-    if (!pools[dev] || ctx == 0 || ctx != ctxs[dev]) {
-        pools[dev] = nullptr;
-        if (ctx == 0) return nullptr;  // contexts cannot be told apart
-        cudaMemPoolProps pr;
-        std::memset(&pr, 0, sizeof(pr));
-        pr.allocType = cudaMemAllocationTypePinned;
-        pr.location.type = cudaMemLocationTypeDevice;
-        pr.location.id = dev;
-        unsigned long long keep = kTablePoolKeep;
-        if (cudaMemPoolCreate(&pools[dev], &pr) != cudaSuccess ||
-            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            pools[dev] = nullptr;
-        }
-        ctxs[dev] = ctx;
+    if (ctx == 0) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    for (const Pool& p : pools)
+        if (p.dev == dev && p.ctx == ctx) return p.pool;
+    cudaMemPoolProps pr;
+    std::memset(&pr, 0, sizeof(pr));
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    unsigned long long keep = kTablePoolKeep;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &pr) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        pool = nullptr;
     }
-    return pools[dev];
+    pools.push_back(Pool{dev, ctx, pool});
+    return pool;
 }
 
 // A table of n doubles on `st`, for the caller to cudaFreeAsync.  Returns
