@@ -461,6 +461,17 @@ __device__ __forceinline__ double rcp1(double s) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
     return fma(r, fma(-s, r, 1.0), r);
 }
+// The FP64 engines' reciprocal of the weight sums: rcp1 (relative error of
+// about 2^-46, times the state's offset from v0), or, FULL, within one ulp.
+// FULL serves the layouts TMA refuses, whose states the per-face kernels gave
+// to full precision before (WENO5-TENO 119x87x103 x 8: 1.7e-16 off the exact
+// states, in norm; 2.5e-17 here, 3.6e-16 with rcp1; 391 against 387 us per
+// x/y/z pass).
+template <bool FULL>
+__device__ __forceinline__ double rcp_sum(double s) {
+    if constexpr (FULL) return nr_rcp(s);
+    return rcp1(s);
+}
 
 // One-sided MP median of an FP64 engine's face (see March64::face), with the
 // side of each state given by the sign of its offset from v0.
@@ -528,12 +539,13 @@ __device__ __forceinline__ bool teno5_keep(double b0, double b1, double b2, doub
 // TENO weights of WENO7 as the reference writes them (f90:1491-1506):
 // beta(4) = eps, tau = |beta(4) - beta(3)|, alpha_q = (1 + tau / beta_q)^6 for
 // q = 0..4, cutoff flags for q = 0..3, and alpha(4) kept in the final sums
-// (returned in a4).  False when the sums leave the reciprocal form's range.
+// (returned in a4; FULL as rcp_sum).  False when the sums leave the reciprocal form's range.
+template <bool FULL>
 __device__ __forceinline__ bool teno7_keep(double b0, double b1, double b2, double b3, double eps, double ct, bool& k0,
                                            bool& k1, bool& k2, bool& k3, double& a4) {
     const double tau = fabs(eps - b3);
     const double t0 = fma(tau, rcp1(b0), 1.0), t1 = fma(tau, rcp1(b1), 1.0), t2 = fma(tau, rcp1(b2), 1.0),
-                 t3 = fma(tau, rcp1(b3), 1.0), t4 = fma(tau, rcp1(eps), 1.0);
+                 t3 = fma(tau, rcp1(b3), 1.0), t4 = fma(tau, rcp_sum<FULL>(eps), 1.0);
     const double x0 = t0 * t0, x1 = t1 * t1, x2 = t2 * t2, x3 = t3 * t3, x4 = t4 * t4;
     const double al0 = x0 * x0 * x0, al1 = x1 * x1 * x1, al2 = x2 * x2 * x2, al3 = x3 * x3 * x3;
     a4 = x4 * x4 * x4;
@@ -544,7 +556,8 @@ __device__ __forceinline__ bool teno7_keep(double b0, double b1, double b2, doub
     return mid_range_prod(s) && mid_range(a4);
 }
 
-struct March64 {
+template <bool FULL>
+struct March64R {
     double vm1, v0, vp1, vp2;   // cells J-1 .. J+2
     double dm2, dm1, d0, dp1;   // d[k] = v[k+1] - v[k], k = J-2 .. J+1
     double s1;                  // d[J+1]^2
@@ -673,7 +686,7 @@ struct March64 {
         mapped_side(a.ucf + 15, a.mcR, a.ucf + 6, P0, P1, P2, ER, GR, ok);
         const double p = GL * GR;
         ok = ok && mid_range_prod(p);
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(EL * GR, r, v0);
         R = fma(ER * GL, r, v0);
         if constexpr (MPF) mp_sided(sign_clear(EL), sign_clear(ER), L, R);
@@ -713,7 +726,7 @@ struct March64 {
         // within the ratio of the ideal weights of each other
         const double p = SL * SR;
         const bool ok = mid_range_prod(p);
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(EL * SR, r, v0);
         R = fma(ER * SL, r, v0);
         if constexpr (MPF) mp_sided(sign_clear(EL), sign_clear(ER), L, R);
@@ -785,13 +798,14 @@ struct March64 {
         // a per-face row marks a face with a negative ideal weight by a NaN in
         // dL(0), which the cutoff may leave out of the sums: test it here
         if constexpr (!std::is_same_v<C, ParamCoefs>) ok = ok && (c.dL(0) == c.dL(0));
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(EL * SR, r, v0);
         R = fma(ER * SL, r, v0);
         if constexpr (MPF) mp_sided(sign_clear(EL), sign_clear(ER), L, R);
         return ok;
     }
 };
+using March64 = March64R<false>;
 
 // The reference sequence for one face (cells o+1 .. o+5 of the column).
 template <bool MPF>
@@ -886,7 +900,8 @@ __global__ void march_face_table7_kernel(CoefPtrs cp, long long nc, int rows, do
     tab[i] = x;
 }
 
-struct March64_7 {
+template <bool FULL>
+struct March64_7R {
     double vm1, v0, vp1, vp2, vp3;        // cells J-1 .. J+3
     double dm3, dm2, dm1, d0, dp1, dp2;    // d[k] = v[k+1] - v[k], k = J-3 .. J+2
     double s1, s2, c12;                    // d[J+1]^2, d[J+2]^2, d[J+1] d[J+2]
@@ -995,7 +1010,7 @@ struct March64_7 {
         const double ER = fma(P0, eR0, fma(P1, eR1, fma(P2, eR2, P3 * eR3)));
         const double p = SL * SR;
         const bool ok = mid_range_prod(p);
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(EL * SR, r, v0);
         R = fma(ER * SL, r, v0);
         if constexpr (MPF) {
@@ -1037,7 +1052,7 @@ struct March64_7 {
     __device__ __forceinline__ bool face_teno(const MarchArgs& a, const C& c, double& L, double& R) const {
         bool k0, k1, k2, k3;
         double a4;
-        const bool ok0 = teno7_keep(B0, B1, B2, B3, a.wp.eps, a.wp.teno_ct, k0, k1, k2, k3, a4);
+        const bool ok0 = teno7_keep<FULL>(B0, B1, B2, B3, a.wp.eps, a.wp.teno_ct, k0, k1, k2, k3, a4);
         const double eL0 = fma(c.kL(0), dm1, fma(c.kL(1), dm2, c.kL(2) * dm3));
         const double eL1 = fma(c.kL(3), d0, fma(c.kL(4), dm1, c.kL(5) * dm2));
         const double eL2 = fma(c.kL(6), dp1, fma(c.kL(7), d0, c.kL(8) * dm1));
@@ -1055,13 +1070,14 @@ struct March64_7 {
         bool ok = ok0 && mid_range_prod(p);
         // a per-face row's NaN mark (negative ideal weight) may be cut from the sums
         if constexpr (!std::is_same_v<C, ParamCoefs7>) ok = ok && (c.dL(0) == c.dL(0));
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(SL, v0, EL) * (DR * r);
         R = fma(SR, v0, ER) * (DL * r);
         if constexpr (MPF) mp64_sided(vm1, v0, vp1, dm1, d0, mA, mB, sign_clear(L - v0), sign_clear(R - v0), L, R);
         return ok;
     }
 };
+using March64_7 = March64_7R<false>;
 // The reference sequence for one WENO7 face with face-dependent
 // coefficients: core face o - 3 of the arrays.
 template <bool MPF>
@@ -1389,7 +1405,7 @@ struct March32_7 {
     __device__ __forceinline__ bool face_teno(const MarchArgs& a, float& L, float& R) const {
         bool k0, k1, k2, k3;
         double a4;
-        const bool ok0 = teno7_keep(B0, B1, B2, B3, a.wp.eps, a.wp.teno_ct, k0, k1, k2, k3, a4);
+        const bool ok0 = teno7_keep<false>(B0, B1, B2, B3, a.wp.eps, a.wp.teno_ct, k0, k1, k2, k3, a4);
         const double aL0 = k0 ? a.ucf[24] : 0.0, aL1 = k1 ? a.ucf[25] : 0.0, aL2 = k2 ? a.ucf[26] : 0.0,
                      aL3 = k3 ? a.ucf[27] : 0.0;
         const double aR0 = k0 ? a.ucf[28] : 0.0, aR1 = k1 ? a.ucf[29] : 0.0, aR2 = k2 ? a.ucf[30] : 0.0,
@@ -1498,7 +1514,8 @@ __global__ void march_face_table3_kernel(CoefPtrs cp, long long nc, int rows, do
     tab[i] = x;
 }
 
-struct March64_3 {
+template <bool FULL>
+struct March64_3R {
     double vm1, v0, vp1, vp2;   // cells J-1 .. J+2
     double dm1, d0, dp1;        // d[J-1], d[J], d[J+1]
     double B0, B1;              // beta_0(J), beta_1(J)
@@ -1550,13 +1567,14 @@ struct March64_3 {
         const double ER = fma(P0, c.kR(0) * d0, P1 * (c.kR(1) * dm1));
         const double p = SL * SR;
         const bool ok = mid_range_prod(p);
-        const double r = rcp1(p);
+        const double r = rcp_sum<FULL>(p);
         L = fma(EL * SR, r, v0);
         R = fma(ER * SL, r, v0);
         if (MPF && core) mp64_sided(vm1, v0, vp1, dm1, d0, mA, mB, sign_clear(EL), sign_clear(ER), L, R);
         return ok;
     }
 };
+using March64_3 = March64_3R<false>;
 
 struct March32_3 {
     float vm1, v0, vp1, vp2;    // cells J-1 .. J+2

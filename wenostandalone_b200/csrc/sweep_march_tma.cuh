@@ -147,10 +147,6 @@ __device__ __forceinline__ unsigned swz(unsigned row, unsigned i) {
     }
 }
 
-template <typename T> struct MarchEngine;
-template <> struct MarchEngine<double> { using type = March64; };
-template <> struct MarchEngine<float> { using type = March32; };
-
 template <bool MPF, bool PF>
 __device__ __forceinline__ void march_redo(const MarchArgs& a, const double* col, long long o, double& L, double& R) {
     if constexpr (PF) march64_redo_faces<MPF>(a, col, o, L, R);
@@ -256,10 +252,13 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     static_assert(!MULTI || !PF, "grouped sweeps: face-independent coefficients");
     constexpr int RW = pf_row_doubles(ORDER), RB = pf_chunk_bytes(ORDER);  // per-face table rows
     static_assert(!TENOW || !PF || ORDER != 3, "TENO with a per-face table: WENO5 / WENO7");
+    // layouts TMA refuses: full reciprocals (rcp_sum), except for WENO5-JS
+    // with face-independent coefficients, whose marching kernel took them
+    constexpr bool FULL = PST && (ORDER != 5 || WS != 0 || PF);
     using Engine = std::conditional_t<
-        ORDER == 7, std::conditional_t<sizeof(T) == 8, March64_7, March32_7>,
-        std::conditional_t<ORDER == 3, std::conditional_t<sizeof(T) == 8, March64_3, March32_3>,
-                           typename MarchEngine<T>::type>>;
+        ORDER == 7, std::conditional_t<sizeof(T) == 8, March64_7R<FULL>, March32_7>,
+        std::conditional_t<ORDER == 3, std::conditional_t<sizeof(T) == 8, March64_3R<FULL>, March32_3>,
+                           std::conditional_t<sizeof(T) == 8, March64R<FULL>, March32>>>;
     constexpr int PUSH0 = ORDER == 7 ? 7 : 6;             // tile position of the cell pushed after face f0
     extern __shared__ __align__(1024) unsigned char smem_mt[];
     unsigned char* base = smem_mt + ((1024u - (smem_u32(smem_mt) & 1023u)) & 1023u);

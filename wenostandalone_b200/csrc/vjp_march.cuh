@@ -134,7 +134,8 @@ struct MarchVjp {
     // TENOW: TENO weights (f90:578-606), d_k delta_k / sum d delta with the
     // cutoff flags delta_k of the forward sequence; the flags are constant
     // between cutoff flips, so the weights pull nothing back to beta.
-    template <bool MPF, bool TENOW>
+    // FULL: reciprocals within one ulp (rcp_sum).
+    template <bool MPF, bool TENOW, bool FULL>
     __device__ __forceinline__ void face(const MarchArgs& a, double gLin, double gRin, int& pick, bool& ok) {
         const March64& w = f;
         ok = beta_ok(w.b0) && beta_ok(w.b1) && beta_ok(w.b2);
@@ -154,7 +155,7 @@ struct MarchVjp {
         const double aL0 = a.ucf[12] * P0, aL1 = a.ucf[13] * P1, aL2 = a.ucf[14] * P2;
         const double aR0 = a.ucf[15] * P0, aR1 = a.ucf[16] * P1, aR2 = a.ucf[17] * P2;
         const double SL = (aL0 + aL1) + aL2, SR = (aR0 + aR1) + aR2;
-        const double r = rcp1(SL * SR), gSL = SR * r, gSR = SL * r;
+        const double r = rcp_sum<FULL>(SL * SR), gSL = SR * r, gSR = SL * r;
         const double wL0 = aL0 * gSL, wL1 = aL1 * gSL, wL2 = aL2 * gSL;
         const double wR0 = aR0 * gSR, wR1 = aR1 * gSR, wR2 = aR2 * gSR;
         // candidate offsets e_k = p_k - v0
@@ -203,7 +204,7 @@ struct MarchVjp {
         const double t1 = fma(gpL1, eL1 - xL, gpR1 * (eR1 - xR));
         const double t2 = fma(gpL2, eL2 - xL, gpR2 * (eR2 - xR));
         const double b12 = B1 * B2, b02 = B0 * B2, b01 = B0 * B1;
-        const double rB = -2.0 * rcp1(B0 * b12);
+        const double rB = -2.0 * rcp_sum<FULL>(B0 * b12);
         const double gb0 = t0 * (rB * b12), gb1 = t1 * (rB * b02), gb2 = t2 * (rB * b01);
         // beta_0 (d0, dp1): b0 dp1^2 + b1 d0 dp1 + b2 d0^2; beta_1 (dm1, d0); beta_2 (dm2, dm1)
         gdp1 = fma(gb0, fma(2.0 * a.ucf[18], w.dp1, a.ucf[19] * w.d0), gdp1);
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
             const double gL = live ? __ldg(t.gLp + oo + 3) : 0.0, gR = live ? __ldg(t.gRp + oo + 3) : 0.0;
             int pk;
             bool ok;
-            m.template face<MPF, TENOW>(a, gL, gR, pk, ok);
+            m.template face<MPF, TENOW, LDR>(a, gL, gR, pk, ok);
             if (pk || (!ok && live)) {
                 // cells 3..9 of the column = J-3 .. J+3 of face 3 (J = 6)
                 double c7[7], acc7[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 const double gR = valid ? cot(kc, 1, i) : 0.0;
                 int pk;
                 bool ok;
-                m.template face<MPF, TENOW>(a, gL, gR, pk, ok);
+                m.template face<MPF, TENOW, LDR>(a, gL, gR, pk, ok);
                 picks |= (unsigned long long)(valid ? pk : 0) << (6 * i);
                 bad |= (ok || !valid) ? 0u : (1u << i);
                 outv[i] = m.advance(a, (i < 2) ? cell(kc, 6 + i) : cell(kc + 1, i - 2)) + oldg(kc, i);
