@@ -1,6 +1,6 @@
 // vjp_march.cuh -- adjoint (VJP) of the FP64 WENO5 (+MP) sweep with JS or
-// TENO weights and face-independent coefficients, marching along the sweep
-// like the forward kernel of sweep_march_tma.cuh.
+// TENO weights, marching along the sweep like the forward kernel of
+// sweep_march_tma.cuh.
 //
 // A warp owns 32 columns and walks a segment of their cells (vjp_march_cut).
 // At face J it recomputes the forward state from the carried window
@@ -38,6 +38,12 @@
 // columns of all cross axes, and the gradient leaves by plain stores or
 // (accumulating) FP64 reductions, whose one add rounds as a load and an add
 // do.
+//
+// PF: face-dependent coefficients.  Every CTA holds the whole table of the
+// sweep (27 coefficients a face) in shared memory, read at warp-uniform
+// addresses; staged per chunk and warp it would not fit beside the tiles.
+// us per x/y/z gradient, 97x80x65 x 5: 689 with one thread per column
+// (vjp_kernel), 574 here.  Bound by FP64 issue with 8 warps an SM.
 #pragma once
 
 #include <cuda.h>
@@ -62,6 +68,7 @@ struct VjpMarchArgs {
     unsigned tx_bytes;  // bytes one stage receives
     const double* gLp;  // cotangents (ns, c1, c2, V)
     const double* gRp;
+    int rows;           // rows of the per-face table
 };
 
 // beta in [2^-100, 2^100): then the one-reciprocal weights, 1/beta and
@@ -107,6 +114,46 @@ __device__ __forceinline__ double mp_pick(double x, double v0, double nb, double
     return s2 ? T1 : B;
 }
 
+// Coefficient sources of one face (Coef<5> order): the kernel parameters, or
+// the face's row of the CTA's table, kVjpRow doubles with a mark at the end
+// (1: a negative or NaN ideal weight; the face is redone from the arrays).
+constexpr int kVjpRow = 28;
+struct VjpParam {
+    const MarchArgs& a;
+    __device__ __forceinline__ double operator()(int q) const { return a.ucf[q]; }
+    __device__ __forceinline__ bool marked() const { return false; }
+};
+struct VjpRow {
+    const double2* p;
+    __device__ __forceinline__ explicit VjpRow(const double* row) : p(reinterpret_cast<const double2*>(row)) {}
+    __device__ __forceinline__ double operator()(int q) const { return (q & 1) ? p[q >> 1].y : p[q >> 1].x; }
+    __device__ __forceinline__ bool marked() const { return p[13].y != 0.0; }
+};
+// Beta coefficients the pair (d[J], d[J+1]) of row's face J enters, stencil r
+// of face J + r (March64::push).
+struct VjpPair {
+    const double* row;
+    __device__ __forceinline__ double b(int q) const { return row[(q / 3) * kVjpRow + 18 + q]; }
+};
+
+// Row f of the table: core face clamp(f - 3) of the arrays.  One thread per
+// entry, as the sweeps' tables.
+__global__ void vjp_face_table_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long f = i / kVjpRow;
+    const int q = (int)(i % kVjpRow);
+    if (f >= rows) return;
+    const long long c = table_core(f, nc);
+    const bool neg = q >= 12 && (q < 18 || q == 27) && table_negative(cp, c, 3);
+    double x;
+    if (q < 6) x = cp.polyL[c + nc * (q / 2 + 5 * (q % 2))];
+    else if (q < 12) x = cp.polyR[c + nc * ((q - 6) / 2 + 5 * (q % 2))];
+    else if (q < 18) x = neg ? 1.0 : (q < 15 ? cp.dL[q - 12 + 5 * c] : cp.dR[q - 15 + 5 * c]);
+    else if (q < 27) x = cp.beta[c + nc * ((q - 18) / 3 + 5 * (q % 3))];
+    else x = neg ? 1.0 : 0.0;
+    tab[i] = x;
+}
+
 struct MarchVjp {
     March64 f;                          // forward window at face J
     double cA1, cA2, cB1, cB2;          // minmod gradients of mA (e2[J-1], e2[J]) and mB (e2[J], e2[J+1])
@@ -116,6 +163,15 @@ struct MarchVjp {
     __device__ __forceinline__ void init(const MarchArgs& a, double c0, double c1, double c2, double c3,
                                          double c4) {
         f.init(a, c0, c1, c2, c3, c4);
+        start(c0, c1, c2, c3);
+    }
+    // row: the row of face J in the table
+    __device__ __forceinline__ void init(const MarchArgs& a, const double* row, double c0, double c1, double c2,
+                                         double c3, double c4) {
+        f.init(a, VjpPair{row - 2 * kVjpRow}, VjpPair{row - kVjpRow}, VjpPair{row}, c0, c1, c2, c3, c4);
+        start(c0, c1, c2, c3);
+    }
+    __device__ __forceinline__ void start(double c0, double c1, double c2, double c3) {
         const double em = (c2 - c1) - (c1 - c0), ez = (c3 - c2) - (c2 - c1);
         mm64_grad(em, ez, cA1, cA2);
         mm64_grad(ez, f.e2, cB1, cB2);
@@ -135,10 +191,10 @@ struct MarchVjp {
     // cutoff flags delta_k of the forward sequence; the flags are constant
     // between cutoff flips, so the weights pull nothing back to beta.
     // FULL: reciprocals within one ulp (rcp_sum).
-    template <bool MPF, bool TENOW, bool FULL>
-    __device__ __forceinline__ void face(const MarchArgs& a, double gLin, double gRin, int& pick, bool& ok) {
+    template <bool MPF, bool TENOW, bool FULL, class C>
+    __device__ __forceinline__ void face(const MarchArgs& a, const C& cf, double gLin, double gRin, int& pick, bool& ok) {
         const March64& w = f;
-        ok = beta_ok(w.b0) && beta_ok(w.b1) && beta_ok(w.b2);
+        ok = beta_ok(w.b0) && beta_ok(w.b1) && beta_ok(w.b2) && !cf.marked();
         const double B0 = ok ? w.b0 : 1.0, B1 = ok ? w.b1 : 1.0, B2 = ok ? w.b2 : 1.0;
         double P0, P1, P2;
         if constexpr (TENOW) {
@@ -152,17 +208,17 @@ struct MarchVjp {
             P0 = q1 * q2; P1 = q0 * q2; P2 = q0 * q1;
         }
         const double gL = ok ? gLin : 0.0, gR = ok ? gRin : 0.0;
-        const double aL0 = a.ucf[12] * P0, aL1 = a.ucf[13] * P1, aL2 = a.ucf[14] * P2;
-        const double aR0 = a.ucf[15] * P0, aR1 = a.ucf[16] * P1, aR2 = a.ucf[17] * P2;
+        const double aL0 = cf(12) * P0, aL1 = cf(13) * P1, aL2 = cf(14) * P2;
+        const double aR0 = cf(15) * P0, aR1 = cf(16) * P1, aR2 = cf(17) * P2;
         const double SL = (aL0 + aL1) + aL2, SR = (aR0 + aR1) + aR2;
         const double r = rcp_sum<FULL>(SL * SR), gSL = SR * r, gSR = SL * r;
         const double wL0 = aL0 * gSL, wL1 = aL1 * gSL, wL2 = aL2 * gSL;
         const double wR0 = aR0 * gSR, wR1 = aR1 * gSR, wR2 = aR2 * gSR;
         // candidate offsets e_k = p_k - v0
-        const double eL0 = fma(a.ucf[1], w.d0, a.ucf[0] * w.dp1), eL1 = fma(a.ucf[3], w.dm1, a.ucf[2] * w.d0),
-                     eL2 = fma(a.ucf[5], w.dm2, a.ucf[4] * w.dm1);
-        const double eR0 = fma(a.ucf[7], w.d0, a.ucf[6] * w.dp1), eR1 = fma(a.ucf[9], w.dm1, a.ucf[8] * w.d0),
-                     eR2 = fma(a.ucf[11], w.dm2, a.ucf[10] * w.dm1);
+        const double eL0 = fma(cf(1), w.d0, cf(0) * w.dp1), eL1 = fma(cf(3), w.dm1, cf(2) * w.d0),
+                     eL2 = fma(cf(5), w.dm2, cf(4) * w.dm1);
+        const double eR0 = fma(cf(7), w.d0, cf(6) * w.dp1), eR1 = fma(cf(9), w.dm1, cf(8) * w.d0),
+                     eR2 = fma(cf(11), w.dm2, cf(10) * w.dm1);
         const double xL = fma(wL0, eL0, fma(wL1, eL1, wL2 * eL2));
         const double xR = fma(wR0, eR0, fma(wR1, eR1, wR2 * eR2));
         double gLw = gL, gRw = gR;
@@ -194,10 +250,10 @@ struct MarchVjp {
         const double gpL0 = gLw * wL0, gpL1 = gLw * wL1, gpL2 = gLw * wL2;
         const double gpR0 = gRw * wR0, gpR1 = gRw * wR1, gpR2 = gRw * wR2;
         gc0 += gLw + gRw;
-        gdp1 = fma(a.ucf[0], gpL0, fma(a.ucf[6], gpR0, gdp1));
-        gd0 = fma(a.ucf[1], gpL0, fma(a.ucf[7], gpR0, fma(a.ucf[2], gpL1, fma(a.ucf[8], gpR1, gd0))));
-        gdm1 = fma(a.ucf[3], gpL1, fma(a.ucf[9], gpR1, fma(a.ucf[4], gpL2, fma(a.ucf[10], gpR2, gdm1))));
-        gdm2 = fma(a.ucf[5], gpL2, fma(a.ucf[11], gpR2, gdm2));
+        gdp1 = fma(cf(0), gpL0, fma(cf(6), gpR0, gdp1));
+        gd0 = fma(cf(1), gpL0, fma(cf(7), gpR0, fma(cf(2), gpL1, fma(cf(8), gpR1, gd0))));
+        gdm1 = fma(cf(3), gpL1, fma(cf(9), gpR1, fma(cf(4), gpL2, fma(cf(10), gpR2, gdm1))));
+        gdm2 = fma(cf(5), gpL2, fma(cf(11), gpR2, gdm2));
         if constexpr (TENOW) return;
         // d out / d beta_k = -2 w_k (e_k - x) / beta_k
         const double t0 = fma(gpL0, eL0 - xL, gpR0 * (eR0 - xR));
@@ -207,24 +263,32 @@ struct MarchVjp {
         const double rB = -2.0 * rcp_sum<FULL>(B0 * b12);
         const double gb0 = t0 * (rB * b12), gb1 = t1 * (rB * b02), gb2 = t2 * (rB * b01);
         // beta_0 (d0, dp1): b0 dp1^2 + b1 d0 dp1 + b2 d0^2; beta_1 (dm1, d0); beta_2 (dm2, dm1)
-        gdp1 = fma(gb0, fma(2.0 * a.ucf[18], w.dp1, a.ucf[19] * w.d0), gdp1);
-        gd0 = fma(gb0, fma(a.ucf[19], w.dp1, 2.0 * a.ucf[20] * w.d0), gd0);
-        gd0 = fma(gb1, fma(2.0 * a.ucf[21], w.d0, a.ucf[22] * w.dm1), gd0);
-        gdm1 = fma(gb1, fma(a.ucf[22], w.d0, 2.0 * a.ucf[23] * w.dm1), gdm1);
-        gdm1 = fma(gb2, fma(2.0 * a.ucf[24], w.dm1, a.ucf[25] * w.dm2), gdm1);
-        gdm2 = fma(gb2, fma(a.ucf[25], w.dm1, 2.0 * a.ucf[26] * w.dm2), gdm2);
+        gdp1 = fma(gb0, fma(2.0 * cf(18), w.dp1, cf(19) * w.d0), gdp1);
+        gd0 = fma(gb0, fma(cf(19), w.dp1, 2.0 * cf(20) * w.d0), gd0);
+        gd0 = fma(gb1, fma(2.0 * cf(21), w.d0, cf(22) * w.dm1), gd0);
+        gdm1 = fma(gb1, fma(cf(22), w.d0, 2.0 * cf(23) * w.dm1), gdm1);
+        gdm1 = fma(gb2, fma(2.0 * cf(24), w.dm1, cf(25) * w.dm2), gdm1);
+        gdm2 = fma(gb2, fma(cf(25), w.dm1, 2.0 * cf(26) * w.dm2), gdm2);
     }
 
     // After face o (centre J): d[J-2] is complete, so is cell J-2; returns
     // cell J-3 (= o) and advances to face o+1 with cell J+3 = n.
     __device__ __forceinline__ double advance(const MarchArgs& a, double n) {
+        return advance([&](March64& w) { w.push(a, n); }, n);
+    }
+    // row: the row of face o + 1 in the table
+    __device__ __forceinline__ double advance(const MarchArgs& a, const double* row, double n) {
+        return advance([&](March64& w) { w.push(a, VjpPair{row}, n); }, n);
+    }
+    template <class Push>
+    __device__ __forceinline__ double advance(const Push& push, double n) {
         gcm1 += gdm2;
         gcm2 -= gdm2;
         const double out = gcm3;
         const double ne2 = (n - f.vp2) - f.dp1;
         double c1, c2;
         mm64_grad(f.e2, ne2, c1, c2);
-        f.push(a, n);
+        push(f);
         cA1 = cB1; cA2 = cB2; cB1 = c1; cB2 = c2;
         gdm2 = gdm1; gdm1 = gd0; gd0 = gdp1; gdp1 = 0.0;
         gcm3 = gcm2; gcm2 = gcm1; gcm1 = gc0; gc0 = gcp1; gcp1 = 0.0;
@@ -281,12 +345,16 @@ __device__ __forceinline__ void route_side(bool left, int code, double g, const 
     }
 }
 
-template <bool MPF, int KIND, bool TENOW, bool LDR>
+// PF: coefficients from the per-face table `tab` of `rows` rows (with LDR,
+// for every layout), which each CTA copies to shared memory: 28 doubles a
+// face, read at warp-uniform addresses.
+template <bool MPF, int KIND, bool TENOW, bool LDR, bool PF>
 __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     vjp_march_kernel(const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tgL,
                      const __grid_constant__ CUtensorMap tgR, const __grid_constant__ CUtensorMap tgo,
                      const __grid_constant__ CUtensorMap tgs, const __grid_constant__ MarchArgs a,
                      const VjpMarchArgs t, double* __restrict__ gv) {
+    static_assert(LDR || !PF, "per-face table: loads by the lanes");
     constexpr int F = kTmaF, S = kVjpStages;
     // column tiles: 34 cells from one left of column 0 (TMA's 16-byte start)
     constexpr int XW = LDR ? 32 : 34, XS = LDR ? 0 : 1;
@@ -309,6 +377,11 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     if (lane == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    double* rows = (double*)(base + (size_t)kVjpWarps * t.warp_bytes + (size_t)kVjpWarps * S * 8);
+    if constexpr (PF) {
+        for (int i = threadIdx.x; i < t.rows * kVjpRow; i += kVjpWarps * 32) rows[i] = __ldg(a.ftab + i);
+        __syncthreads();
     }
     __syncwarp();
     const long long nwarps = (long long)gridDim.x * kVjpWarps;
@@ -397,12 +470,25 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
         return *(const double*)(gstage(k) + arr * 2048 + swz<double>((unsigned)lane, (unsigned)i));
     };
     // generic pull-back of face o on the cells c7 = J-3 .. J+3
-    auto redo = [&](const double* c7, double gL, double gR, double* acc7) {
+    auto redo = [&](int o, const double* c7, double gL, double gR, double* acc7) {
         Coef<5> cf;
-        for (int q = 0; q < 6; ++q) { cf.pL[q] = a.ucf[q]; cf.pR[q] = a.ucf[6 + q]; }
-        for (int q = 0; q < 3; ++q) { cf.dL[q] = a.ucf[12 + q]; cf.dR[q] = a.ucf[15 + q]; }
-        for (int q = 0; q < 9; ++q) cf.b[q] = a.ucf[18 + q];
+        if constexpr (PF) {
+            cf.load(a.cp.polyL, a.cp.polyR, a.cp.dL, a.cp.dR, a.cp.beta, a.nc, table_core(o, a.nc));
+        } else {
+            for (int q = 0; q < 6; ++q) { cf.pL[q] = a.ucf[q]; cf.pR[q] = a.ucf[6 + q]; }
+            for (int q = 0; q < 3; ++q) { cf.dL[q] = a.ucf[12 + q]; cf.dR[q] = a.ucf[15 + q]; }
+            for (int q = 0; q < 9; ++q) cf.b[q] = a.ucf[18 + q];
+        }
         face_vjp<5>(c7 + 3, cf, TENOW ? TENO : JS, a.wp.eps, a.wp.teno_ct, MPF, gL, gR, acc7);
+    };
+    // the pull-back of face o, and the step to face o + 1 with cell n
+    auto face = [&](MarchVjp& m, int o, double gL, double gR, int& pk, bool& ok) {
+        if constexpr (PF) m.template face<MPF, TENOW, LDR>(a, VjpRow(rows + o * kVjpRow), gL, gR, pk, ok);
+        else m.template face<MPF, TENOW, LDR>(a, VjpParam{a}, gL, gR, pk, ok);
+    };
+    auto advance = [&](MarchVjp& m, int o, double n) -> double {
+        if constexpr (PF) return m.advance(a, rows + (o + 1) * kVjpRow, n);
+        else return m.advance(a, n);
     };
 
     for (long long item = (long long)blockIdx.x * kVjpWarps + warp; item < a.n_items && !failed; item += nwarps) {
@@ -462,20 +548,23 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
         if (live && !t.acc && sg == 0)
             for (int q = 0; q < 4; ++q) gcol[q * a.sJ] = 0.0;
         MarchVjp m;
-        m.init(a, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
+        const int ob = 3 + F * cb;
+        if constexpr (PF)
+            m.init(a, rows + ob * kVjpRow, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
+        else m.init(a, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
         if (cb == 0) {
             // face 3 (a later segment's reaches only cells of the
             // chunk it does not write)
             const double gL = live ? __ldg(t.gLp + oo + 3) : 0.0, gR = live ? __ldg(t.gRp + oo + 3) : 0.0;
             int pk;
             bool ok;
-            m.template face<MPF, TENOW, LDR>(a, gL, gR, pk, ok);
+            face(m, 3, gL, gR, pk, ok);
             if (pk || (!ok && live)) {
                 // cells 3..9 of the column = J-3 .. J+3 of face 3 (J = 6)
                 double c7[7], acc7[7] = {0, 0, 0, 0, 0, 0, 0};
                 for (int q = 0; q < 7; ++q) c7[q] = __ldg(col + (3 + q) * a.sJ);
                 if (!ok) {
-                    redo(c7, gL, gR, acc7);
+                    redo(3, c7, gL, gR, acc7);
                 } else {
                     route_side(true, pk & 7, gL, c7 + 1, acc7 + 1);
                     route_side(false, pk >> 3, gR, c7 + 1, acc7 + 1);
@@ -489,7 +578,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 m.gdp1 += acc7[5];
             }
         }
-        (void)m.advance(a, cell(k0, 5));  // cell f0 - 1: not written here
+        (void)advance(m, ob, cell(k0, 5));  // cell f0 - 1: not written here
         // chunk c: faces f0 .. f0+7 (f0 = 4 + 8 (cb + c)); face f0+i pushes cell
         // f0+i+6 = stage c position 6+i (i < 2) or stage c+1 position i-2,
         // and emits cell f0+i = position i of stage c's tiles
@@ -515,10 +604,10 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 const double gR = valid ? cot(kc, 1, i) : 0.0;
                 int pk;
                 bool ok;
-                m.template face<MPF, TENOW, LDR>(a, gL, gR, pk, ok);
+                face(m, o, gL, gR, pk, ok);
                 picks |= (unsigned long long)(valid ? pk : 0) << (6 * i);
                 bad |= (ok || !valid) ? 0u : (1u << i);
-                outv[i] = m.advance(a, (i < 2) ? cell(kc, 6 + i) : cell(kc + 1, i - 2)) + oldg(kc, i);
+                outv[i] = advance(m, o, (i < 2) ? cell(kc, 6 + i) : cell(kc + 1, i - 2)) + oldg(kc, i);
             }
             if (__any_sync(0xffffffffu, picks != 0ull || bad != 0u)) {
                 // (the area is the row tiles' outgoing tile too; its last store
@@ -539,7 +628,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                     }
                     const double gL = cot(kc, 0, i), gR = cot(kc, 1, i);
                     if (again) {
-                        redo(c7, gL, gR, acc7);
+                        redo(f0 + i, c7, gL, gR, acc7);
                     } else {
                         route_side(true, pk & 7, gL, c7 + 1, acc7 + 1);
                         route_side(false, pk >> 3, gR, c7 + 1, acc7 + 1);
@@ -639,17 +728,29 @@ inline void vjp_march_cut(MarchArgs& a, long long tiles, long long warps) {
 }
 
 // Host side: the marching adjoint for FP64 WENO5 with JS or TENO weights and
-// face-independent coefficients.  TMA staging when every base and row is a
-// 16-byte multiple, copies by the lanes otherwise.  Returns 1003 (unsupported) for sweeps of fewer than
-// 8 faces or a lane axis the march arguments did not choose; the caller then
+// face-independent coefficients (ucf), or with the per-face table tab built
+// from cp (the lanes then load in every layout).  TMA staging when every base
+// and row is a 16-byte multiple, copies by the lanes otherwise.  Returns 1003
+// (unsupported) for sweeps of fewer than 8 faces or a lane axis the march arguments did not choose; the caller then
 // runs vjp_kernel.  gv must already hold what is to be added to when acc is
 // set.
+// Rows of the per-face table (the last chunk's last face reads the pairs of
+// three rows after its own), and the most for which it fits into shared
+// memory beside the warps' tiles (227 KB in all: sweeps of up to 214 faces);
+// longer sweeps take vjp_kernel.
+inline long long vjp_table_rows(const SweepGeom& g) { return (g.ns + 1) / kTmaF * kTmaF + 15; }
+constexpr int kVjpLdrWarpBytes = (kVjpStages * (4096 + 2048) + 13 * 32 * 8 + 2 * 32 * 8 + 511) / 512 * 512;
+constexpr long long kVjpMaxRows =
+    (227 * 1024 - 1024 - kVjpWarps * (kVjpLdrWarpBytes + kVjpStages * 8)) / (kVjpRow * 8);
 inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, bool acc,
-                            const double* v, const double* ucf, const WenoParams& wp, const double* gL,
-                            const double* gR, double* gv, cudaStream_t st, int sms) {
-    EncodeTiledFn enc = encode_tiled_fn();
+                            const double* v, const double* ucf, const double* tab, const CoefPtrs& cp,
+                            const WenoParams& wp, const double* gL, const double* gR, double* gv, cudaStream_t st,
+                            int sms) {
+    const EncodeTiledFn enc = tab ? nullptr : encode_tiled_fn();
     if (g.ns < 8 || g.nc < 1) return 1003;
     MarchArgs a = make_march_args(g, v, nullptr, nullptr, wp, ucf);
+    a.ftab = tab;
+    a.cp = cp;
     VjpMarchArgs t{};
     const bool kind1 = folded && dir != 0;
     if (kind1 != (a.sU == 1)) return 1003;
@@ -711,19 +812,19 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
     } else {
         t.stage_bytes = 2048;
     }
-    t.warp_bytes = kVjpStages * (4096 + t.stage_bytes) + 13 * 32 * 8;
-    if (!tma) t.warp_bytes += 2 * 32 * 8;
-    t.warp_bytes = (t.warp_bytes + 511) / 512 * 512;
-    const size_t smem = 1024 + (size_t)kVjpWarps * t.warp_bytes + (size_t)kVjpWarps * kVjpStages * 8;
+    t.warp_bytes = tma ? (kVjpStages * (4096 + t.stage_bytes) + 13 * 32 * 8 + 511) / 512 * 512 : kVjpLdrWarpBytes;
+    t.rows = tab ? (int)vjp_table_rows(g) : 0;
+    const size_t smem = (size_t)t.rows * kVjpRow * 8 + 1024 + (size_t)kVjpWarps * t.warp_bytes + (size_t)kVjpWarps * kVjpStages * 8;
     using KFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, VjpMarchArgs,
                          double*);
 #define WSB_VJP_ROW(MPF, TENOW)                                                      \
-    {{vjp_march_kernel<MPF, 0, TENOW, false>, vjp_march_kernel<MPF, 1, TENOW, false>}, \
-     {vjp_march_kernel<MPF, 0, TENOW, true>, vjp_march_kernel<MPF, 1, TENOW, true>}}
-    static const KFn table[2][2][2][2] = {{WSB_VJP_ROW(false, false), WSB_VJP_ROW(true, false)},
+    {{vjp_march_kernel<MPF, 0, TENOW, false, false>, vjp_march_kernel<MPF, 1, TENOW, false, false>}, \
+     {vjp_march_kernel<MPF, 0, TENOW, true, false>, vjp_march_kernel<MPF, 1, TENOW, true, false>},   \
+     {vjp_march_kernel<MPF, 0, TENOW, true, true>, vjp_march_kernel<MPF, 1, TENOW, true, true>}}
+    static const KFn table[2][2][3][2] = {{WSB_VJP_ROW(false, false), WSB_VJP_ROW(true, false)},
                                           {WSB_VJP_ROW(false, true), WSB_VJP_ROW(true, true)}};
 #undef WSB_VJP_ROW
-    const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][tma ? 0 : 1][kind1 ? 1 : 0];
+    const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][tma ? 0 : (tab ? 2 : 1)][kind1 ? 1 : 0];
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kVjpWarps * 32, smem);

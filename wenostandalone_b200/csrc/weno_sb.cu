@@ -569,9 +569,25 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
     const bool uni = ucf != nullptr;
     if (uni && order == 5 && (gr->scheme == WENO_SB_JS || gr->scheme == WENO_SB_TENO) && kernel_choice() != 1 &&
         march_weights_ok(ucf)) {
-        int rc = launch_vjp_march(d.E, a.g, dir, folded, a.mp != 0, a.accumulate != 0, v, ucf, a.wp, gL, gR, gv, st,
-                                  num_sms());
+        int rc = launch_vjp_march(d.E, a.g, dir, folded, a.mp != 0, a.accumulate != 0, v, ucf, nullptr, cp, a.wp, gL,
+                                  gR, gv, st, num_sms());
         if (rc != WENO_SB_ERR_UNSUPPORTED) return rc == 0 ? cuda_err(cudaGetLastError(), "vjp march launch") : rc;
+    }
+    // coefficient arrays: the marching adjoint with a per-face table, where it
+    // fits (us per x/y/z gradient, 97x80x65 x 5: 574; vjp_kernel 689)
+    if (!uni && order == 5 && (gr->scheme == WENO_SB_JS || gr->scheme == WENO_SB_TENO) && kernel_choice() != 1 &&
+        a.g.ns >= 8 && vjp_table_rows(a.g) <= kVjpMaxRows) {
+        const int rows = (int)vjp_table_rows(a.g);
+        double* tab = nullptr;
+        int rc = table_alloc(&tab, (size_t)rows * kVjpRow, st);
+        if (rc == 0) {
+            vjp_face_table_kernel<<<(unsigned)((rows * kVjpRow + 127) / 128), 128, 0, st>>>(cp, a.g.nc, rows, tab);
+            rc = launch_vjp_march(d.E, a.g, dir, folded, a.mp != 0, a.accumulate != 0, v, nullptr, tab, cp, a.wp, gL,
+                                  gR, gv, st, num_sms());
+            const cudaError_t le = cudaGetLastError(), fe = cudaFreeAsync(tab, st);
+            if (rc == 0) return cuda_err(le != cudaSuccess ? le : fe, "vjp march launch (per-face table)");
+        }
+        if (rc != WENO_SB_ERR_UNSUPPORTED) return rc;
     }
     using KFn = void (*)(VjpArgs);
     static const KFn table[3][2][2] = {
