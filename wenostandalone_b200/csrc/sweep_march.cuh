@@ -461,11 +461,11 @@ __device__ __forceinline__ double rcp1(double s) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
     return fma(r, fma(-s, r, 1.0), r);
 }
-// The FP64 engines' reciprocal of the weight sums: rcp1 (relative error of
-// about 2^-46, times the state's offset from v0), or, FULL, within one ulp.
-// FULL serves the layouts TMA refuses, whose states the per-face kernels gave
+// The FP64 engines' reciprocal of the weight sums and the TENO ratios: rcp1
+// (relative error of about 2^-46; in the sums, times the state's offset from
+// v0), or, FULL, within one ulp.  FULL serves the layouts TMA refuses, whose states the per-face kernels gave
 // to full precision before (WENO5-TENO 119x87x103 x 8: 1.7e-16 off the exact
-// states, in norm; 2.5e-17 here, 3.6e-16 with rcp1; 391 against 387 us per
+// states, in norm; 2.5e-17 here, 3.6e-16 with rcp1; 396 against 387 us per
 // x/y/z pass).
 template <bool FULL>
 __device__ __forceinline__ double rcp_sum(double s) {
@@ -524,34 +524,50 @@ __device__ __forceinline__ void mp32_sided(float fm1, float f0, float mA, float 
 // TENO weights of WENO5 (f90:578-606) for betas b0..b2: the cutoff flags
 // (alpha_k / sum alpha >= CT, alpha_k = (1 + tau / beta_k)^6,
 // tau = |beta_2 - beta_0|); false when the alpha sum leaves [1, 2^996)
-// (a zero beta, or ratios past 10^50).
+// (a zero beta, or ratios past 10^50).  FULL: ratios as rcp_sum, compared
+// with CT times the sum, so that a flag falls where the divisions put it but
+// for a few ulp of the cutoff (one Newton step per reciprocal leaves 2^-43).
+template <bool FULL>
 __device__ __forceinline__ bool teno5_keep(double b0, double b1, double b2, double ct, bool& k0, bool& k1, bool& k2) {
     const double tau = fabs(b2 - b0);
-    const double t0 = fma(tau, rcp1(b0), 1.0), t1 = fma(tau, rcp1(b1), 1.0), t2 = fma(tau, rcp1(b2), 1.0);
+    const double t0 = fma(tau, rcp_sum<FULL>(b0), 1.0), t1 = fma(tau, rcp_sum<FULL>(b1), 1.0),
+                 t2 = fma(tau, rcp_sum<FULL>(b2), 1.0);
     const double x0 = t0 * t0, x1 = t1 * t1, x2 = t2 * t2;
     const double al0 = x0 * x0 * x0, al1 = x1 * x1 * x1, al2 = x2 * x2 * x2;
     const double s = (al0 + al1) + al2;
-    const double rs = rcp1(s);
-    k0 = !(al0 * rs < ct); k1 = !(al1 * rs < ct); k2 = !(al2 * rs < ct);
+    if constexpr (FULL) {
+        const double cut = ct * s;
+        k0 = !(al0 < cut); k1 = !(al1 < cut); k2 = !(al2 < cut);
+    } else {
+        const double rs = rcp1(s);
+        k0 = !(al0 * rs < ct); k1 = !(al1 * rs < ct); k2 = !(al2 * rs < ct);
+    }
     return mid_range_prod(s);
 }
 
 // TENO weights of WENO7 as the reference writes them (f90:1491-1506):
 // beta(4) = eps, tau = |beta(4) - beta(3)|, alpha_q = (1 + tau / beta_q)^6 for
 // q = 0..4, cutoff flags for q = 0..3, and alpha(4) kept in the final sums
-// (returned in a4; FULL as rcp_sum).  False when the sums leave the reciprocal form's range.
+// (returned in a4; FULL as teno5_keep).  False when the sums leave the
+// reciprocal form's range.
 template <bool FULL>
 __device__ __forceinline__ bool teno7_keep(double b0, double b1, double b2, double b3, double eps, double ct, bool& k0,
                                            bool& k1, bool& k2, bool& k3, double& a4) {
     const double tau = fabs(eps - b3);
-    const double t0 = fma(tau, rcp1(b0), 1.0), t1 = fma(tau, rcp1(b1), 1.0), t2 = fma(tau, rcp1(b2), 1.0),
-                 t3 = fma(tau, rcp1(b3), 1.0), t4 = fma(tau, rcp_sum<FULL>(eps), 1.0);
+    const double t0 = fma(tau, rcp_sum<FULL>(b0), 1.0), t1 = fma(tau, rcp_sum<FULL>(b1), 1.0),
+                 t2 = fma(tau, rcp_sum<FULL>(b2), 1.0),
+                 t3 = fma(tau, rcp_sum<FULL>(b3), 1.0), t4 = fma(tau, rcp_sum<FULL>(eps), 1.0);
     const double x0 = t0 * t0, x1 = t1 * t1, x2 = t2 * t2, x3 = t3 * t3, x4 = t4 * t4;
     const double al0 = x0 * x0 * x0, al1 = x1 * x1 * x1, al2 = x2 * x2 * x2, al3 = x3 * x3 * x3;
     a4 = x4 * x4 * x4;
     const double s = ((al0 + al1) + (al2 + al3)) + a4;
-    const double rs = rcp1(s);
-    k0 = !(al0 * rs < ct); k1 = !(al1 * rs < ct); k2 = !(al2 * rs < ct); k3 = !(al3 * rs < ct);
+    if constexpr (FULL) {
+        const double cut = ct * s;
+        k0 = !(al0 < cut); k1 = !(al1 < cut); k2 = !(al2 < cut); k3 = !(al3 < cut);
+    } else {
+        const double rs = rcp1(s);
+        k0 = !(al0 * rs < ct); k1 = !(al1 * rs < ct); k2 = !(al2 * rs < ct); k3 = !(al3 * rs < ct);
+    }
     // a4 >= 1; (S + a4)^2 must stay below 2^996 for the final reciprocal
     return mid_range_prod(s) && mid_range(a4);
 }
@@ -776,15 +792,24 @@ struct March64R {
     template <bool MPF, class C>
     __device__ __forceinline__ bool face_teno(const MarchArgs& a, const C& c, double& L, double& R) {
         const double tau = fabs(b2 - b0);
-        const double t0 = fma(tau, rcp1(b0), 1.0), t1 = fma(tau, rcp1(b1), 1.0), t2 = fma(tau, rcp1(b2), 1.0);
+        const double t0 = fma(tau, rcp_sum<FULL>(b0), 1.0), t1 = fma(tau, rcp_sum<FULL>(b1), 1.0),
+                 t2 = fma(tau, rcp_sum<FULL>(b2), 1.0);
         const double x0 = t0 * t0, x1 = t1 * t1, x2 = t2 * t2;
         const double al0 = x0 * x0 * x0, al1 = x1 * x1 * x1, al2 = x2 * x2 * x2;
         const double s = (al0 + al1) + al2;
         // s >= 1 (every alpha is); below 2^996 its reciprocal and the
         // products with it stay normal (NaN and inf fail the test too)
         const bool s_ok = mid_range_prod(s);
-        const double rs = rcp1(s), ct = a.wp.teno_ct;
-        const bool k0 = !(al0 * rs < ct), k1 = !(al1 * rs < ct), k2 = !(al2 * rs < ct);
+        const double ct = a.wp.teno_ct;
+        bool k0, k1, k2;
+        if constexpr (FULL) {
+            // (as teno5_keep)
+            const double cut = ct * s;
+            k0 = !(al0 < cut); k1 = !(al1 < cut); k2 = !(al2 < cut);
+        } else {
+            const double rs = rcp1(s);
+            k0 = !(al0 * rs < ct); k1 = !(al1 * rs < ct); k2 = !(al2 * rs < ct);
+        }
         const double eL0 = fma(c.kL(1), d0, c.kL(0) * dp1), eL1 = fma(c.kL(3), dm1, c.kL(2) * d0),
                      eL2 = fma(c.kL(5), dm2, c.kL(4) * dm1);
         const double eR0 = fma(c.kR(1), d0, c.kR(0) * dp1), eR1 = fma(c.kR(3), dm1, c.kR(2) * d0),
@@ -1239,7 +1264,7 @@ struct March32 {
     template <bool MPF>
     __device__ __forceinline__ bool face_teno(const MarchArgs& a, float& L, float& R) const {
         bool k0, k1, k2;
-        const bool ok0 = teno5_keep(b0, b1, b2, a.wp.teno_ct, k0, k1, k2);
+        const bool ok0 = teno5_keep<false>(b0, b1, b2, a.wp.teno_ct, k0, k1, k2);
         const double aL0 = k0 ? a.ucf[12] : 0.0, aL1 = k1 ? a.ucf[13] : 0.0, aL2 = k2 ? a.ucf[14] : 0.0;
         const double aR0 = k0 ? a.ucf[15] : 0.0, aR1 = k1 ? a.ucf[16] : 0.0, aR2 = k2 ? a.ucf[17] : 0.0;
         const double SL = (aL0 + aL1) + aL2, SR = (aR0 + aR1) + aR2;

@@ -199,7 +199,7 @@ struct MarchVjp {
         double P0, P1, P2;
         if constexpr (TENOW) {
             bool k0, k1, k2;
-            ok = teno5_keep(B0, B1, B2, a.wp.teno_ct, k0, k1, k2) && ok;
+            ok = teno5_keep<FULL>(B0, B1, B2, a.wp.teno_ct, k0, k1, k2) && ok;
             P0 = k0 ? 1.0 : 0.0;
             P1 = k1 ? 1.0 : 0.0;
             P2 = k2 ? 1.0 : 0.0;
