@@ -260,6 +260,12 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         std::conditional_t<ORDER == 3, std::conditional_t<sizeof(T) == 8, March64_3R<FULL>, March32_3>,
                            std::conditional_t<sizeof(T) == 8, March64R<FULL>, March32>>>;
     constexpr int PUSH0 = ORDER == 7 ? 7 : 6;             // tile position of the cell pushed after face f0
+    // WENO3: the outer cells of a face reach it through the limiter's
+    // curvatures alone, to which mm64 gives NaN no special treatment, so the
+    // faces of a chunk that a NaN or infinite cell may reach are redone (zero
+    // times every cell, one operation a face; the other families' weights see
+    // every cell of the limiter)
+    constexpr bool NANC = FULL && MPF && ORDER == 3;
     extern __shared__ __align__(1024) unsigned char smem_mt[];
     unsigned char* base = smem_mt + ((1024u - (smem_u32(smem_mt) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -559,6 +565,10 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             else
                 w.init(a, cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4), cell(k0, 5));
         }
+        bool dirty = false;  // NANC: such a cell among the last pushed
+        if constexpr (NANC)
+            dirty = !(0.0 * (((double)cell(k0, 1) + cell(k0, 2)) + ((double)cell(k0, 3) + cell(k0, 4)) + cell(k0, 5)) ==
+                      0.0);
         // chunk c: faces f0 .. f0+7 (f0 = f_start + 8c), pushes cells
         // f0+6 .. f0+13 = positions 6, 7 of tile c and 0 .. 5 of tile c+1
         for (int c = 0; c < nch; ++c) {
@@ -581,6 +591,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             // moves whole 16-byte chunks), column-tile cells one by one
             constexpr int G = 16 / (int)sizeof(T);
             T Lg[G], Rg[G], cg[G];
+            double z = 0.0;
 #pragma unroll
             for (int i = 0; i < F; ++i) {
                 const int q = PUSH0 + i;                  // position of the pushed cell, tiles c / c+1
@@ -633,12 +644,18 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 T n;
                 if constexpr (KIND == 0) n = cg[pq % G];
                 else n = cell(kq, pq);
+                if constexpr (NANC) z = fma((double)n, 0.0, z);
                 if constexpr (PF && ORDER == 7) w.push(a, Row7{srow(kc, i + 1)}, n);
                 else if constexpr (PF && ORDER == 3) w.push(a, Row3{srow(kc, i + 1)}, n);
                 else if constexpr (PF) w.push(a, BetaRow(srow(kc, i + 1)), n);
                 else w.push(a, n);
             }
             const int nF = f_end - f0 < F ? f_end - f0 : F;
+            if constexpr (NANC) {
+                const bool now = !(z == 0.0);
+                if (now || dirty) bad = ~0u;
+                dirty = now;
+            }
             bad &= (1u << nF) - 1u;
             if (bad) {
                 const T* col = column(u0, wv, vv);
