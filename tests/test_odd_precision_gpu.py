@@ -1,15 +1,47 @@
 """Layouts that TMA refuses keep the precision of the one-thread-per-face
-kernels: TENO cutoffs fall on the side on which the divisions put them."""
+kernels: FP32 storage of the families those computed in FP64 (WENO3-JS and
+the TENO weights) rounds once, and TENO cutoffs fall on the side on which the
+divisions put them."""
 import numpy as np
 import pytest
 
-from gpu_util import to_dev
+from gpu_util import from_dev, to_dev
 
 pytestmark = pytest.mark.gpu
 
 # Nd = cells + 2 buff + 1 = 33, 35, 31: no direction's rows are multiples of
 # 4 floats or of 2 doubles
 M, N, P, BUFF = 20, 22, 18, 6
+
+
+@pytest.mark.parametrize("order,scheme", [(3, 0), (5, 3), (7, 3)])
+def test_fp32_storage_rounds_once(oracle_mod, order, scheme):
+    """Without the limiter a state is the FP64 state rounded to FP32: within
+    half an ulp, 2^-24 of its size, of the oracle, plus the FP64 bar."""
+    import torch
+    import wenostandalone_b200 as wsb
+    from wenostandalone_b200 import api, fields
+    # (the reference's WENO7-TENO has alpha(4) = (1 + tau / eps)^6, which cuts
+    # every stencil at the usual eps)
+    eps = 0.05 if order == 7 else 1e-16
+    g = wsb.Grid(M, N, P, 2, BUFF, scheme=scheme, weno_eps=eps)
+    rng = np.random.default_rng(6)
+    vf = rng.standard_normal((M + 19, N + 19, P + 19, 2)).astype(np.float32).astype(np.float64)
+    vf = np.asfortranarray(vf)
+    for d in range(3):
+        coefs = fields.uniform_weno_coefficients(order, g.nc(d))
+        rs = oracle_mod.reshape(vf, M, N, P, BUFF, d)
+        ref = oracle_mod.order1_copy(vf, M, N, P, BUFF, d)
+        got = [to_dev(x, torch.float32) for x in ref]
+        oracle_mod.reconstruct(rs, coefs, order, scheme=scheme, eps=eps, vL=ref[0], vR=ref[1])
+        api.weno_uniform(g, d, order, to_dev(rs, torch.float32), coefs, *got)
+        sure = np.ones(ref[0].shape, dtype=bool)
+        if scheme == 3:
+            sure = oracle_mod.teno_margin(rs, coefs, order, eps=eps) > 1e-10
+            assert sure.mean() > 0.99
+        for x, r in zip(got, ref):
+            e = np.abs(from_dev(x, g.face_shape(d)) - r)
+            assert np.all((e <= 2.0 ** -24 * np.abs(r) + 1e-12 * np.abs(r).max())[sure]), (d, e[sure].max())
 
 
 def _omega(x, order, coefs, eps):

@@ -84,6 +84,15 @@ __host__ __device__ constexpr int mtma_stages(bool pf, bool pst) { return pst ? 
 __host__ __device__ constexpr int mtma_outs(bool pf, bool pst, int order, int es) {
     return pst ? kPstOut : (pf ? kPfOut : (order == 3 && es == 8 ? 1 : kTmaOut));
 }
+// FP32 storage in layouts whose rows are not 16-byte multiples: the FP64
+// engine for WENO3-JS and for TENO weights, which the one-thread-per-face
+// kernels computed in FP64 before, with one rounding.  us per sweep of 163
+// cells, 125 x 151 columns x 8, on those kernels / with the FP32 engine (whose
+// weights and sums are FP32) / here: WENO3 240 / 135 / 193, WENO5-TENO 856 /
+// 207 / 262, WENO7-TENO 2250 / 277 / 385.
+__host__ __device__ constexpr bool mtma_wide(bool pst, int order, int ws, int es) {
+    return pst && es == 4 && (order == 3 || ws == 3);
+}
 // rows f0 .. f0 + 8 of a chunk (WENO5 / WENO7 table rows)
 __host__ __device__ constexpr int pf_row_doubles(int order) {
     return order == 7 ? kFaceRow7 : (order == 3 ? kFaceRow3 : kFaceRow);
@@ -255,10 +264,14 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
     // layouts TMA refuses: full reciprocals (rcp_sum), except for WENO5-JS
     // with face-independent coefficients, whose marching kernel took them
     constexpr bool FULL = PST && (ORDER != 5 || WS != 0 || PF);
+    // FP32 storage, engine in FP64 (mtma_wide): the states are rounded as they
+    // are stored
+    constexpr bool E64 = sizeof(T) == 8 || (!MULTI && mtma_wide(PST, ORDER, WS, (int)sizeof(T)));
+    using CT = std::conditional_t<E64, double, T>;
     using Engine = std::conditional_t<
-        ORDER == 7, std::conditional_t<sizeof(T) == 8, March64_7R<FULL>, March32_7>,
-        std::conditional_t<ORDER == 3, std::conditional_t<sizeof(T) == 8, March64_3R<FULL>, March32_3>,
-                           std::conditional_t<sizeof(T) == 8, March64R<FULL>, March32>>>;
+        ORDER == 7, std::conditional_t<E64, March64_7R<FULL>, March32_7>,
+        std::conditional_t<ORDER == 3, std::conditional_t<E64, March64_3R<FULL>, March32_3>,
+                           std::conditional_t<E64, March64R<FULL>, March32>>>;
     constexpr int PUSH0 = ORDER == 7 ? 7 : 6;             // tile position of the cell pushed after face f0
     // WENO3: the outer cells of a face reach it through the limiter's
     // curvatures alone, to which mm64 gives NaN no special treatment, so the
@@ -502,7 +515,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
         Engine w;
         if (sg == 0 && ORDER != 3) {
             // face 3 (cells 4..8 = tile positions 0..4), plain stores
-            T L, R;
+            CT L, R;
             bool ok;
             if constexpr (ORDER == 7) {
                 // face 3 reads cells 3 .. 9: cell 3 lies before tile 0 (cells 4 .. 11)
@@ -538,14 +551,20 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 // (the redo sequences take the weights and strides from the
                 // sweep's arguments)
                 if constexpr (ORDER == 7 && PF) march64_7_redo_faces<MPF>(ga(), column(u0, wv, vv), 3, L, R);
-                else if constexpr (ORDER == 7) march7_redo<MPF>(ga(), column(u0, wv, vv), 3, L, R);
+                else if constexpr (!std::is_same_v<CT, T>) {
+                    T Lr, Rr;
+                    if constexpr (ORDER == 7) march7_redo<MPF>(ga(), column(u0, wv, vv), 3, Lr, Rr);
+                    else march_redo<MPF, PF>(ga(), column(u0, wv, vv), 3, Lr, Rr);
+                    L = Lr;
+                    R = Rr;
+                } else if constexpr (ORDER == 7) march7_redo<MPF>(ga(), column(u0, wv, vv), 3, L, R);
                 else march_redo<MPF, PF>(ga(), column(u0, wv, vv), 3, L, R);
             }
             if (live) {
                 const long long oi =
                     3 + (PST ? offs[lane] : (long long)(u0 + lane) * g.oU + wv * g.oW + vv * g.oV);
-                outL[oi] = L;
-                outR[oi] = R;
+                outL[oi] = (T)L;
+                outR[oi] = (T)R;
             }
             if constexpr (ORDER == 7 && PF) w.push(a, Row7{row(4)}, cell(k0, 6));
             else if constexpr (ORDER == 7) w.push(a, cell(k0, 6));
@@ -610,7 +629,7 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                         }
                     }
                 }
-                T L, R;
+                CT L, R;
                 bool ok;
                 if constexpr (ORDER == 3 && PF)
                     ok = w.template face<MPF>(a, Row3{srow(kc, i)}, L, R, f0 + i >= 3 && f0 + i <= o_last - 4);
@@ -625,8 +644,8 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
                 else if constexpr (WS == 1) ok = w.template face_mapped<MPF>(a, L, R);
                 else ok = w.template face<MPF>(a, L, R);
                 if (!ok) bad |= 1u << i;
-                Lg[i % G] = L;
-                Rg[i % G] = R;
+                Lg[i % G] = (T)L;
+                Rg[i % G] = (T)R;
                 if (NOUT == 1 && i == G - 1 && wait_out) {
                     if (lane == 0) bulk_wait_read0();
                     __syncwarp();
@@ -772,17 +791,19 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
 #ifndef WSB_MTMA_MIN_BLOCKS_W7
 #define WSB_MTMA_MIN_BLOCKS_W7 2  // WENO7 carries ~27 doubles of state: 3 CTAs per SM would spill
 #endif
-// CTAs per SM by order (WENO3: 4, but 3 with plain stores, whose second
-// output tile leaves no shared memory for a fourth)
-template <int ORDER, typename T, bool PST>
+// CTAs per SM by order (WENO3: 4, but 3 with plain stores from the FP64
+// engine: its second output tile leaves no shared memory for a fourth, and
+// storing FP32 its registers do not fit)
+template <int ORDER, typename T, bool PST, bool E64 = sizeof(T) == 8>
 constexpr int kMtmaMinBlocks = ORDER == 7 ? WSB_MTMA_MIN_BLOCKS_W7
-                               : ORDER == 3 && !(PST && sizeof(T) == 8)
+                               : ORDER == 3 && !(PST && E64)
                                    ? 4
                                    : (sizeof(T) == 8 ? WSB_MTMA_MIN_BLOCKS : WSB_MTMA_MIN_BLOCKS_F32);
 
 // One sweep: maps and arguments in the parameter bank.
 template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER = 5, int WS = 0, bool PST = false>
-__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST>))
+__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST, sizeof(T) == 8 ||
+                                                                  mtma_wide(PST, ORDER, WS, (int)sizeof(T))>))
     sweep_march_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap toutL,
                            const __grid_constant__ CUtensorMap toutR, const __grid_constant__ MarchArgs a,
                            const MarchTmaArgs t) {
