@@ -5,7 +5,8 @@ same finite values."""
 import numpy as np
 import pytest
 
-from gpu_util import to_dev
+from gpu_util import from_dev, rel_err, to_dev
+from test_adjoint_gpu import TOL_AD
 from test_parity_gpu import varying_coefficients
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,62 @@ def test_sweeps(monkeypatch, order, scheme, entry, bad):
             out.append((L, R))
         for got, ref in zip(*out):
             _same(got, ref, 1e-12)
+
+
+def _gradients(monkeypatch, wsb, g, d, entry, vf, c, gL, gR, g0, mp=True):
+    from wenostandalone_b200 import api
+    out = []
+    flags = wsb.F_FOLDED | wsb.F_ACCUMULATE | (wsb.F_MP if mp else 0)
+    for kernel in ("auto", "generic"):
+        monkeypatch.setenv("WENO_SB_KERNEL", kernel)
+        gv = to_dev(g0)
+        cs = tuple(c) if entry == "uniform" else tuple(to_dev(a) for a in c)
+        api.vjp(g, d, 5, to_dev(vf), cs, to_dev(gL), to_dev(gR), gv, flags=flags, uniform=entry == "uniform")
+        out.append(gv)
+    return out
+
+
+@pytest.mark.parametrize("cells", [(20, 22, 18), (21, 23, 19)])  # odd rows; rows that suit TMA
+@pytest.mark.parametrize("scale", [2.0 ** -600, 2.0 ** -300, 2.0 ** 300])
+@pytest.mark.parametrize("entry", ["uniform", "arrays"])
+@pytest.mark.parametrize("scheme", [0, 3])
+def test_scaled_ideal_weights(scheme, entry, scale, cells):
+    """The weights are normalised, so a common factor of the ideal weights
+    changes nothing."""
+    import wenostandalone_b200 as wsb
+    from wenostandalone_b200 import api, fields
+    m, n, p = cells
+    g = wsb.Grid(m, n, p, 1, BUFF, scheme=scheme)
+    vf = fields.sinusoid_shock_field(m, n, p, 1, BUFF, seed=4, shock=False)
+    rng = np.random.default_rng(5)
+    for d in range(3):
+        gL, gR = (to_dev(rng.standard_normal(g.face_shape(d))) for _ in range(2))
+        out = []
+        for f in (1.0, scale):
+            c = _coefs(wsb, entry, 5, g, d)
+            c[2] *= f
+            c[3] *= f
+            cs = tuple(c) if entry == "uniform" else tuple(to_dev(a) for a in c)
+            gv = to_dev(np.zeros(vf.shape))
+            api.vjp(g, d, 5, to_dev(vf), cs, gL, gR, gv, flags=wsb.F_FOLDED | wsb.F_MP, uniform=entry == "uniform")
+            out.append(from_dev(gv, vf.shape))
+        assert rel_err(out[1], out[0]) <= TOL_AD, d
+
+
+@pytest.mark.parametrize("entry", ["uniform", "arrays"])
+@pytest.mark.parametrize("zero", [0, 1, 2])
+def test_teno_zero_ideal_weight(monkeypatch, entry, zero):
+    """A face whose kept stencils have no weight on one side has NaN there
+    only, as with the divisions."""
+    import wenostandalone_b200 as wsb
+    from wenostandalone_b200 import fields
+    g = wsb.Grid(M, N, P, 2, BUFF, scheme=3)
+    vf = fields.smooth_jump_field(M, N, P, 2, BUFF, seed=5)
+    rng = np.random.default_rng(12)
+    for d in range(3):
+        gL, gR = rng.standard_normal(g.face_shape(d)), rng.standard_normal(g.face_shape(d))
+        c = _coefs(wsb, entry, 5, g, d)
+        c[2][zero] = 0.0
+        c[3][2 - zero] = 0.0
+        got, ref = _gradients(monkeypatch, wsb, g, d, entry, vf, c, gL, gR, np.zeros(vf.shape))
+        _same(got, ref, 100 * TOL_AD)

@@ -114,9 +114,22 @@ __device__ __forceinline__ double mp_pick(double x, double v0, double nb, double
     return s2 ? T1 : B;
 }
 
+// Whether the three ideal weights of one side suit the one-reciprocal form
+// with betas in [2^-100, 2^100): each 0 or within [2^-60, 2^60], so that the
+// product of both sides' sums stays within 2^(+-920), and not all 0; TENO:
+// none 0, as the cutoff may keep a stencil without weight alone.  (Not so:
+// negative and NaN weights, which the limiter's one-sided median does not
+// take either.)
+__host__ __device__ inline bool vjp_side_ok(double d0, double d1, double d2, bool teno) {
+    const double lo = 0x1p-60, hi = 0x1p60;
+    auto one = [&](double x) { return (x >= lo && x <= hi) || (x == 0.0 && !teno); };
+    return one(d0) && one(d1) && one(d2) && d0 + d1 + d2 > 0.0;
+}
+
 // Coefficient sources of one face (Coef<5> order): the kernel parameters, or
 // the face's row of the CTA's table, kVjpRow doubles with a mark at the end
-// (1: a negative or NaN ideal weight; the face is redone from the arrays).
+// (1: ideal weights that are not vjp_side_ok; the face is redone from the
+// arrays).
 constexpr int kVjpRow = 28;
 struct VjpParam {
     const MarchArgs& a;
@@ -138,19 +151,20 @@ struct VjpPair {
 
 // Row f of the table: core face clamp(f - 3) of the arrays.  One thread per
 // entry, as the sweeps' tables.
-__global__ void vjp_face_table_kernel(CoefPtrs cp, long long nc, int rows, double* __restrict__ tab) {
+__global__ void vjp_face_table_kernel(CoefPtrs cp, long long nc, int rows, bool teno, double* __restrict__ tab) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long f = i / kVjpRow;
     const int q = (int)(i % kVjpRow);
     if (f >= rows) return;
     const long long c = table_core(f, nc);
-    const bool neg = q >= 12 && (q < 18 || q == 27) && table_negative(cp, c, 3);
+    auto side = [&](const double* p) { return vjp_side_ok(p[5 * c], p[5 * c + 1], p[5 * c + 2], teno); };
+    const bool mark = q >= 12 && (q < 18 || q == 27) && !(side(cp.dL) && side(cp.dR));
     double x;
     if (q < 6) x = cp.polyL[c + nc * (q / 2 + 5 * (q % 2))];
     else if (q < 12) x = cp.polyR[c + nc * ((q - 6) / 2 + 5 * (q % 2))];
-    else if (q < 18) x = neg ? 1.0 : (q < 15 ? cp.dL[q - 12 + 5 * c] : cp.dR[q - 15 + 5 * c]);
+    else if (q < 18) x = mark ? 1.0 : (q < 15 ? cp.dL[q - 12 + 5 * c] : cp.dR[q - 15 + 5 * c]);
     else if (q < 27) x = cp.beta[c + nc * ((q - 18) / 3 + 5 * (q % 3))];
-    else x = neg ? 1.0 : 0.0;
+    else x = mark ? 1.0 : 0.0;
     tab[i] = x;
 }
 

@@ -567,8 +567,9 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
     if (folded && !acc_flag)
         WSB_CUDA(cudaMemsetAsync(gv, 0, sizeof(double) * d.E[0] * d.E[1] * d.E[2] * d.nv, st));
     const bool uni = ucf != nullptr;
-    if (uni && order == 5 && (gr->scheme == WENO_SB_JS || gr->scheme == WENO_SB_TENO) && kernel_choice() != 1 &&
-        march_weights_ok(ucf)) {
+    const bool teno = gr->scheme == WENO_SB_TENO;
+    if (uni && order == 5 && (gr->scheme == WENO_SB_JS || teno) && kernel_choice() != 1 &&
+        vjp_side_ok(ucf[12], ucf[13], ucf[14], teno) && vjp_side_ok(ucf[15], ucf[16], ucf[17], teno)) {
         int rc = launch_vjp_march(d.E, a.g, dir, folded, a.mp != 0, a.accumulate != 0, v, ucf, nullptr, cp, a.wp, gL,
                                   gR, gv, st, num_sms());
         if (rc != WENO_SB_ERR_UNSUPPORTED) return rc == 0 ? cuda_err(cudaGetLastError(), "vjp march launch") : rc;
@@ -578,13 +579,14 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
     // into a stream capture, where the table would be memory of the graph
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool direct = uni || (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone);
-    if (!uni && direct && order == 5 && (gr->scheme == WENO_SB_JS || gr->scheme == WENO_SB_TENO) && kernel_choice() != 1 &&
+    if (!uni && direct && order == 5 && (gr->scheme == WENO_SB_JS || teno) && kernel_choice() != 1 &&
         a.g.ns >= 8 && vjp_table_rows(a.g) <= kVjpMaxRows) {
         const int rows = (int)vjp_table_rows(a.g);
         double* tab = nullptr;
         int rc = table_alloc(&tab, (size_t)rows * kVjpRow, st);
         if (rc == 0) {
-            vjp_face_table_kernel<<<(unsigned)((rows * kVjpRow + 127) / 128), 128, 0, st>>>(cp, a.g.nc, rows, tab);
+            vjp_face_table_kernel<<<(unsigned)((rows * kVjpRow + 127) / 128), 128, 0, st>>>(cp, a.g.nc, rows, teno,
+                                                                                            tab);
             rc = launch_vjp_march(d.E, a.g, dir, folded, a.mp != 0, a.accumulate != 0, v, nullptr, tab, cp, a.wp, gL,
                                   gR, gv, st, num_sms());
             const cudaError_t le = cudaGetLastError(), fe = cudaFreeAsync(tab, st);
