@@ -75,6 +75,28 @@ def _gradients(monkeypatch, wsb, g, d, entry, vf, c, gL, gR, g0, mp=True):
     return out
 
 
+@pytest.mark.parametrize("where,bad", [("cell", np.nan), ("cell", np.inf), ("cell", 1e200), ("cotangent", np.nan),
+                                       ("cotangent", np.inf), ("gradient", np.nan), ("gradient", np.inf)])
+@pytest.mark.parametrize("entry", ["uniform", "arrays"])
+@pytest.mark.parametrize("scheme", [0, 3])
+def test_adjoint(monkeypatch, scheme, entry, where, bad):
+    import wenostandalone_b200 as wsb
+    from wenostandalone_b200 import fields
+    g = wsb.Grid(M, N, P, 2, BUFF, scheme=scheme)
+    for d in range(3):
+        for mp in (False, True):
+            rng = np.random.default_rng(12)
+            vf = fields.smooth_jump_field(M, N, P, 2, BUFF, seed=5)
+            gL, gR = rng.standard_normal(g.face_shape(d)), rng.standard_normal(g.face_shape(d))
+            g0 = rng.standard_normal(vf.shape)
+            for a in {"cell": [vf], "cotangent": [gL, gR], "gradient": [g0]}[where]:
+                _put(a, bad, 4, 25)
+            c = _coefs(wsb, entry, 5, g, d)
+            got, ref = _gradients(monkeypatch, wsb, g, d, entry, vf, c, gL, gR, g0, mp)
+            # gradients of rough cells reach some hundreds: TOL_AD of that
+            _same(got, ref, 100 * TOL_AD)
+
+
 @pytest.mark.parametrize("cells", [(20, 22, 18), (21, 23, 19)])  # odd rows; rows that suit TMA
 @pytest.mark.parametrize("scale", [2.0 ** -600, 2.0 ** -300, 2.0 ** 300])
 @pytest.mark.parametrize("entry", ["uniform", "arrays"])

@@ -71,6 +71,10 @@ struct VjpMarchArgs {
     int rows;           // rows of the per-face table
 };
 
+__device__ __forceinline__ bool finite_bits(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+
 // beta in [2^-100, 2^100): then the one-reciprocal weights, 1/beta and
 // their products stay normal (an integer test on the exponent field).
 __device__ __forceinline__ bool beta_ok(double b) {
@@ -204,11 +208,16 @@ struct MarchVjp {
     // TENOW: TENO weights (f90:578-606), d_k delta_k / sum d delta with the
     // cutoff flags delta_k of the forward sequence; the flags are constant
     // between cutoff flips, so the weights pull nothing back to beta.
-    // FULL: reciprocals within one ulp (rcp_sum).
+    // FULL (layouts and coefficients that vjp_kernel served before):
+    // reciprocals within one ulp (rcp_sum); a face whose cotangents are not
+    // finite is redone too, and no difference that is not finite enters the
+    // sums of a face that is, so NaN and infinities reach the cells that the
+    // generic pull-back sends them to and no others.
     template <bool MPF, bool TENOW, bool FULL, class C>
     __device__ __forceinline__ void face(const MarchArgs& a, const C& cf, double gLin, double gRin, int& pick, bool& ok) {
         const March64& w = f;
         ok = beta_ok(w.b0) && beta_ok(w.b1) && beta_ok(w.b2) && !cf.marked();
+        if constexpr (FULL) ok = ok && finite_bits(gLin) && finite_bits(gRin);
         const double B0 = ok ? w.b0 : 1.0, B1 = ok ? w.b1 : 1.0, B2 = ok ? w.b2 : 1.0;
         double P0, P1, P2;
         if constexpr (TENOW) {
@@ -222,6 +231,8 @@ struct MarchVjp {
             P0 = q1 * q2; P1 = q0 * q2; P2 = q0 * q1;
         }
         const double gL = ok ? gLin : 0.0, gR = ok ? gRin : 0.0;
+        const bool use = !FULL || ok;
+        const double dm2 = use ? w.dm2 : 0.0, dm1 = use ? w.dm1 : 0.0, d0 = use ? w.d0 : 0.0, dp1 = use ? w.dp1 : 0.0;
         const double aL0 = cf(12) * P0, aL1 = cf(13) * P1, aL2 = cf(14) * P2;
         const double aR0 = cf(15) * P0, aR1 = cf(16) * P1, aR2 = cf(17) * P2;
         const double SL = (aL0 + aL1) + aL2, SR = (aR0 + aR1) + aR2;
@@ -229,10 +240,10 @@ struct MarchVjp {
         const double wL0 = aL0 * gSL, wL1 = aL1 * gSL, wL2 = aL2 * gSL;
         const double wR0 = aR0 * gSR, wR1 = aR1 * gSR, wR2 = aR2 * gSR;
         // candidate offsets e_k = p_k - v0
-        const double eL0 = fma(cf(1), w.d0, cf(0) * w.dp1), eL1 = fma(cf(3), w.dm1, cf(2) * w.d0),
-                     eL2 = fma(cf(5), w.dm2, cf(4) * w.dm1);
-        const double eR0 = fma(cf(7), w.d0, cf(6) * w.dp1), eR1 = fma(cf(9), w.dm1, cf(8) * w.d0),
-                     eR2 = fma(cf(11), w.dm2, cf(10) * w.dm1);
+        const double eL0 = fma(cf(1), d0, cf(0) * dp1), eL1 = fma(cf(3), dm1, cf(2) * d0),
+                     eL2 = fma(cf(5), dm2, cf(4) * dm1);
+        const double eR0 = fma(cf(7), d0, cf(6) * dp1), eR1 = fma(cf(9), dm1, cf(8) * d0),
+                     eR2 = fma(cf(11), dm2, cf(10) * dm1);
         const double xL = fma(wL0, eL0, fma(wL1, eL1, wL2 * eL2));
         const double xR = fma(wR0, eR0, fma(wR1, eR1, wR2 * eR2));
         double gLw = gL, gRw = gR;
@@ -277,12 +288,12 @@ struct MarchVjp {
         const double rB = -2.0 * rcp_sum<FULL>(B0 * b12);
         const double gb0 = t0 * (rB * b12), gb1 = t1 * (rB * b02), gb2 = t2 * (rB * b01);
         // beta_0 (d0, dp1): b0 dp1^2 + b1 d0 dp1 + b2 d0^2; beta_1 (dm1, d0); beta_2 (dm2, dm1)
-        gdp1 = fma(gb0, fma(2.0 * cf(18), w.dp1, cf(19) * w.d0), gdp1);
-        gd0 = fma(gb0, fma(cf(19), w.dp1, 2.0 * cf(20) * w.d0), gd0);
-        gd0 = fma(gb1, fma(2.0 * cf(21), w.d0, cf(22) * w.dm1), gd0);
-        gdm1 = fma(gb1, fma(cf(22), w.d0, 2.0 * cf(23) * w.dm1), gdm1);
-        gdm1 = fma(gb2, fma(2.0 * cf(24), w.dm1, cf(25) * w.dm2), gdm1);
-        gdm2 = fma(gb2, fma(cf(25), w.dm1, 2.0 * cf(26) * w.dm2), gdm2);
+        gdp1 = fma(gb0, fma(2.0 * cf(18), dp1, cf(19) * d0), gdp1);
+        gd0 = fma(gb0, fma(cf(19), dp1, 2.0 * cf(20) * d0), gd0);
+        gd0 = fma(gb1, fma(2.0 * cf(21), d0, cf(22) * dm1), gd0);
+        gdm1 = fma(gb1, fma(cf(22), d0, 2.0 * cf(23) * dm1), gdm1);
+        gdm1 = fma(gb2, fma(2.0 * cf(24), dm1, cf(25) * dm2), gdm1);
+        gdm2 = fma(gb2, fma(cf(25), dm1, 2.0 * cf(26) * dm2), gdm2);
     }
 
     // After face o (centre J): d[J-2] is complete, so is cell J-2; returns
@@ -380,13 +391,15 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     // 512-aligned for the swizzle), the field (and old-gradient) tiles of
     // the S stages, then one area that holds the per-lane corrections of a
     // chunk and afterwards (row tiles) the outgoing [32 u][8 cells] tile;
-    // LDR: the columns' offsets in the field and in the cotangents
+    // LDR: the columns' offsets in the field and in the cotangents, and what
+    // the redone first core face adds to the first chunk
     unsigned char* gring = wbase;
     unsigned char* vring = wbase + S * 4096;
     unsigned char* obuf = wbase + S * 4096 + S * t.stage_bytes;   // t.stage_bytes: v (+ old) per stage
     double* slot = (double*)obuf;  // 13 cells f0 .. f0+12 x 32 lanes
     long long* offs = (long long*)(obuf + 13 * 32 * 8);
     long long* offo = offs + 32;
+    double* first = (double*)(offo + 32);
     unsigned long long* bars = (unsigned long long*)(base + (size_t)kVjpWarps * t.warp_bytes) + warp * S;
     if (lane == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
@@ -566,6 +579,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
         if constexpr (PF)
             m.init(a, rows + ob * kVjpRow, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
         else m.init(a, cell(k0, 0), cell(k0, 1), cell(k0, 2), cell(k0, 3), cell(k0, 4));
+        if constexpr (LDR) first[lane] = 0.0;
         if (cb == 0) {
             // face 3 (a later segment's reaches only cells of the
             // chunk it does not write)
@@ -583,13 +597,19 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                     route_side(true, pk & 7, gL, c7 + 1, acc7 + 1);
                     route_side(false, pk >> 3, gR, c7 + 1, acc7 + 1);
                 }
-                // acc7[q] is cell J-3+q; pending: J-3 .. J+1, and J+2 through d[J+1]
+                // acc7[q] is cell J-3+q; pending: J-3 .. J+1, and J+2 through
+                // d[J+1] (LDR: with the first chunk, whose cell f0 + 4 it is)
                 m.gcm3 += acc7[0];
                 m.gcm2 += acc7[1];
                 m.gcm1 += acc7[2];
                 m.gc0 += acc7[3];
-                m.gcp1 += acc7[4] + acc7[5];
-                m.gdp1 += acc7[5];
+                if constexpr (LDR) {
+                    m.gcp1 += acc7[4];
+                    first[lane] = acc7[5];
+                } else {
+                    m.gcp1 += acc7[4] + acc7[5];
+                    m.gdp1 += acc7[5];
+                }
             }
         }
         (void)advance(m, ob, cell(k0, 5));  // cell f0 - 1: not written here
@@ -623,6 +643,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
                 bad |= (ok || !valid) ? 0u : (1u << i);
                 outv[i] = advance(m, o, (i < 2) ? cell(kc, 6 + i) : cell(kc + 1, i - 2)) + oldg(kc, i);
             }
+            if (LDR && c == 0) outv[4] += first[lane];
             if (__any_sync(0xffffffffu, picks != 0ull || bad != 0u)) {
                 // (the area is the row tiles' outgoing tile too; its last store
                 // has been read: waited at the start of the chunk)
@@ -753,7 +774,7 @@ inline void vjp_march_cut(MarchArgs& a, long long tiles, long long warps) {
 // memory beside the warps' tiles (227 KB in all: sweeps of up to 214 faces);
 // longer sweeps take vjp_kernel.
 inline long long vjp_table_rows(const SweepGeom& g) { return (g.ns + 1) / kTmaF * kTmaF + 15; }
-constexpr int kVjpLdrWarpBytes = (kVjpStages * (4096 + 2048) + 13 * 32 * 8 + 2 * 32 * 8 + 511) / 512 * 512;
+constexpr int kVjpLdrWarpBytes = (kVjpStages * (4096 + 2048) + 13 * 32 * 8 + 3 * 32 * 8 + 511) / 512 * 512;
 constexpr long long kVjpMaxRows =
     (227 * 1024 - 1024 - kVjpWarps * (kVjpLdrWarpBytes + kVjpStages * 8)) / (kVjpRow * 8);
 inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, bool acc,
