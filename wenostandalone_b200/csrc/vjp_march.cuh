@@ -773,10 +773,11 @@ inline void vjp_march_cut(MarchArgs& a, long long tiles, long long warps) {
 // three rows after its own), and the most for which it fits into shared
 // memory beside the warps' tiles (227 KB in all: sweeps of up to 214 faces);
 // longer sweeps take vjp_kernel.
+constexpr int kVjpMaxSmem = 227 * 1024;
 inline long long vjp_table_rows(const SweepGeom& g) { return (g.ns + 1) / kTmaF * kTmaF + 15; }
 constexpr int kVjpLdrWarpBytes = (kVjpStages * (4096 + 2048) + 13 * 32 * 8 + 3 * 32 * 8 + 511) / 512 * 512;
 constexpr long long kVjpMaxRows =
-    (227 * 1024 - 1024 - kVjpWarps * (kVjpLdrWarpBytes + kVjpStages * 8)) / (kVjpRow * 8);
+    (kVjpMaxSmem - 1024 - kVjpWarps * (kVjpLdrWarpBytes + kVjpStages * 8)) / (kVjpRow * 8);
 inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, bool acc,
                             const double* v, const double* ucf, const double* tab, const CoefPtrs& cp,
                             const WenoParams& wp, const double* gL, const double* gR, double* gv, cudaStream_t st,
@@ -860,10 +861,14 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
                                           {WSB_VJP_ROW(false, true), WSB_VJP_ROW(true, true)}};
 #undef WSB_VJP_ROW
     const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][tma ? 0 : (tab ? 2 : 1)][kind1 ? 1 : 0];
-    cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // always the same limit: the size differs from call to call, and another
+    // thread's call must not lower it between here and the launch
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kVjpWarps * 32, smem);
-    if (occ < 1) return 1003;
+    if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kVjpMaxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kVjpWarps * 32, smem) != cudaSuccess || occ < 1) {
+        cudaGetLastError();
+        return 1003;
+    }
     const long long cap = (long long)sms * occ;
     vjp_march_cut(a, tma ? (long long)a.n_ut * a.Nw * a.NV : (a.n_cols + 31) / 32, cap * kVjpWarps);
     const long long blocks = std::min((a.n_items + kVjpWarps - 1) / kVjpWarps, cap);
