@@ -188,7 +188,8 @@ int weno_sb_order1_dev(const weno_sb_grid *g, int dir, int dtype, const double *
  * v_vf when flags has WENO_SB_F_FOLDED.  Per-face coefficient arrays take a
  * per-face table, allocated and freed stream-ordered on `stream` (from a
  * pool of the library that keeps at most 64 MB per device; within a stream
- * capture, by the graph). */
+ * capture, by the graph, except for fields from an 8-byte boundary, which
+ * are captured with kernels that need no table). */
 int weno_sb_weno_dev(const weno_sb_grid *g, int dir, int order, unsigned flags, int dtype,
                      const void *v_in, const weno_sb_coefs *coefs, void *vL, void *vR,
                      void *stream);
@@ -210,7 +211,11 @@ int weno_sb_weno_uniform_dev(const weno_sb_grid *g, int dir, int order, unsigned
  * layout of v_rs_ws, or of v_vf with WENO_SB_F_FOLDED.  gv is overwritten
  * (the cells no face reads get 0) unless WENO_SB_F_ACCUMULATE adds into it,
  * so the three folded sweeps can sum into one gv.  Coefficients come either
- * per face (coefs) or face-independent (face); pass exactly one.  FP64. */
+ * per face (coefs) or face-independent (face); pass exactly one.  FP64.
+ * Per-face WENO5 sweeps of up to 214 faces take a table from the same pool,
+ * as weno_sb_weno_dev; longer ones, and every call within a stream capture,
+ * run a kernel without one (no memory of the graph, and results equal up to
+ * rounding). */
 int weno_sb_vjp_dev(const weno_sb_grid *g, int dir, int order, unsigned flags, const double *v_in,
                     const weno_sb_coefs *coefs, const weno_sb_face_coefs *face, const double *gL,
                     const double *gR, double *gv, void *stream);

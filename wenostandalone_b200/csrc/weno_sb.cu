@@ -384,6 +384,13 @@ cudaMemPool_t table_pool() {
     return pool;
 }
 
+// Whether memory allocated on `st` would belong to a graph (or the stream's
+// state cannot be read).
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
 // A table of n doubles on `st`, for the caller to cudaFreeAsync.  Returns
 // WENO_SB_ERR_UNSUPPORTED when no stream-ordered allocation (or no memory)
 // is available: the caller falls back to the kernels that need no table.
@@ -393,9 +400,7 @@ int table_alloc(double** tab, size_t n, cudaStream_t st) {
     const cudaError_t pending = cudaPeekAtLastError();
     if (pending != cudaSuccess) return cuda_err(cudaGetLastError(), "error pending before the per-face table");
     // (in a capture the memory belongs to the graph, and no pool is made)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool direct = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-    const cudaMemPool_t pool = direct ? table_pool() : nullptr;
+    const cudaMemPool_t pool = capturing(st) ? nullptr : table_pool();
     const cudaError_t ae = pool ? cudaMallocFromPoolAsync((void**)tab, sizeof(double) * n, pool, st)
                                 : cudaMallocAsync((void**)tab, sizeof(double) * n, st);
     if (ae == cudaSuccess) return WENO_SB_OK;
@@ -420,6 +425,10 @@ int launch_march_faces(const long long E[3], const SweepGeom& g, int dir, bool f
                        int ws = 0, int order = 5) {
     if (!cp.polyL || !cp.polyR || !cp.dL || !cp.dR || !cp.beta) return WENO_SB_ERR_UNSUPPORTED;
     if (g.ns < 8) return WENO_SB_ERR_UNSUPPORTED;
+    // (a graph with memory of its own cannot be cloned, made a child graph or
+    // run by two executables at once; fields from an 8-byte boundary are
+    // captured without, by the kernels that need no table)
+    if (((uintptr_t)in & 15) && capturing(st)) return WENO_SB_ERR_UNSUPPORTED;
     const int rows = (int)g.ns + 16;
     double* tab = nullptr;
     const int arc = table_alloc(&tab, (size_t)rows * pf_row_doubles(order), st);
@@ -577,10 +586,8 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
     // coefficient arrays: the marching adjoint with a per-face table, where it
     // fits (us per x/y/z gradient, 97x80x65 x 5: 574; vjp_kernel 689), but not
     // into a stream capture, where the table would be memory of the graph
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool direct = uni || (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone);
-    if (!uni && direct && order == 5 && (gr->scheme == WENO_SB_JS || teno) && kernel_choice() != 1 &&
-        a.g.ns >= 8 && vjp_table_rows(a.g) <= kVjpMaxRows) {
+    if (!uni && order == 5 && (gr->scheme == WENO_SB_JS || teno) && kernel_choice() != 1 &&
+        a.g.ns >= 8 && vjp_table_rows(a.g) <= kVjpMaxRows && !capturing(st)) {
         const int rows = (int)vjp_table_rows(a.g);
         double* tab = nullptr;
         int rc = table_alloc(&tab, (size_t)rows * kVjpRow, st);
