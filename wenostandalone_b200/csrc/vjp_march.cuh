@@ -43,7 +43,7 @@
 // sweep (27 coefficients a face) in shared memory, read at warp-uniform
 // addresses; staged per chunk and warp it would not fit beside the tiles.
 // us per x/y/z gradient, 97x80x65 x 5: 689 with one thread per column
-// (vjp_kernel), 574 here.  Bound by FP64 issue with 8 warps an SM.
+// (vjp_kernel), 561 here.  Bound by FP64 issue with 8 warps an SM.
 #pragma once
 
 #include <cuda.h>
@@ -69,6 +69,10 @@ struct VjpMarchArgs {
     const double* gLp;  // cotangents (ns, c1, c2, V)
     const double* gRp;
     int rows;           // rows of the per-face table
+    // 2 beta_coef of the squares (ucf 18, 20, 21, 23, 24, 26), exact; formed in
+    // the kernel they took registers or an operation a face (832 against 802
+    // us per x/y/z gradient, 128^3 x 5)
+    double b2[6];
 };
 
 __device__ __forceinline__ bool finite_bits(double x) {
@@ -135,15 +139,20 @@ __host__ __device__ inline bool vjp_side_ok(double d0, double d1, double d2, boo
 // (1: ideal weights that are not vjp_side_ok; the face is redone from the
 // arrays).
 constexpr int kVjpRow = 28;
+// Coef<5> index of the k-th square's coefficient (VjpMarchArgs::b2)
+__host__ __device__ constexpr int vjp_square(int k) { return 18 + 3 * (k / 2) + 2 * (k % 2); }
 struct VjpParam {
     const MarchArgs& a;
+    const double* b2;
     __device__ __forceinline__ double operator()(int q) const { return a.ucf[q]; }
+    __device__ __forceinline__ double twice(int k) const { return b2[k]; }
     __device__ __forceinline__ bool marked() const { return false; }
 };
 struct VjpRow {
     const double2* p;
     __device__ __forceinline__ explicit VjpRow(const double* row) : p(reinterpret_cast<const double2*>(row)) {}
     __device__ __forceinline__ double operator()(int q) const { return (q & 1) ? p[q >> 1].y : p[q >> 1].x; }
+    __device__ __forceinline__ double twice(int k) const { return 2.0 * (*this)(vjp_square(k)); }
     __device__ __forceinline__ bool marked() const { return p[13].y != 0.0; }
 };
 // Beta coefficients the pair (d[J], d[J+1]) of row's face J enters, stencil r
@@ -174,25 +183,21 @@ __global__ void vjp_face_table_kernel(CoefPtrs cp, long long nc, int rows, bool 
 
 struct MarchVjp {
     March64 f;                          // forward window at face J
-    double cA1, cA2, cB1, cB2;          // minmod gradients of mA (e2[J-1], e2[J]) and mB (e2[J], e2[J+1])
     double gdm2, gdm1, gd0, gdp1;       // pending gradients of d[J-2] .. d[J+1]
     double gcm3, gcm2, gcm1, gc0, gcp1; // pending gradients of cells J-3 .. J+1
 
     __device__ __forceinline__ void init(const MarchArgs& a, double c0, double c1, double c2, double c3,
                                          double c4) {
         f.init(a, c0, c1, c2, c3, c4);
-        start(c0, c1, c2, c3);
+        start();
     }
     // row: the row of face J in the table
     __device__ __forceinline__ void init(const MarchArgs& a, const double* row, double c0, double c1, double c2,
                                          double c3, double c4) {
         f.init(a, VjpPair{row - 2 * kVjpRow}, VjpPair{row - kVjpRow}, VjpPair{row}, c0, c1, c2, c3, c4);
-        start(c0, c1, c2, c3);
+        start();
     }
-    __device__ __forceinline__ void start(double c0, double c1, double c2, double c3) {
-        const double em = (c2 - c1) - (c1 - c0), ez = (c3 - c2) - (c2 - c1);
-        mm64_grad(em, ez, cA1, cA2);
-        mm64_grad(ez, f.e2, cB1, cB2);
+    __device__ __forceinline__ void start() {
         gdm2 = gdm1 = gd0 = gdp1 = 0.0;
         gcm3 = gcm2 = gcm1 = gc0 = gcp1 = 0.0;
     }
@@ -288,33 +293,29 @@ struct MarchVjp {
         const double rB = -2.0 * rcp_sum<FULL>(B0 * b12);
         const double gb0 = t0 * (rB * b12), gb1 = t1 * (rB * b02), gb2 = t2 * (rB * b01);
         // beta_0 (d0, dp1): b0 dp1^2 + b1 d0 dp1 + b2 d0^2; beta_1 (dm1, d0); beta_2 (dm2, dm1)
-        gdp1 = fma(gb0, fma(2.0 * cf(18), dp1, cf(19) * d0), gdp1);
-        gd0 = fma(gb0, fma(cf(19), dp1, 2.0 * cf(20) * d0), gd0);
-        gd0 = fma(gb1, fma(2.0 * cf(21), d0, cf(22) * dm1), gd0);
-        gdm1 = fma(gb1, fma(cf(22), d0, 2.0 * cf(23) * dm1), gdm1);
-        gdm1 = fma(gb2, fma(2.0 * cf(24), dm1, cf(25) * dm2), gdm1);
-        gdm2 = fma(gb2, fma(cf(25), dm1, 2.0 * cf(26) * dm2), gdm2);
+        gdp1 = fma(gb0, fma(cf.twice(0), dp1, cf(19) * d0), gdp1);
+        gd0 = fma(gb0, fma(cf(19), dp1, cf.twice(1) * d0), gd0);
+        gd0 = fma(gb1, fma(cf.twice(2), d0, cf(22) * dm1), gd0);
+        gdm1 = fma(gb1, fma(cf(22), d0, cf.twice(3) * dm1), gdm1);
+        gdm1 = fma(gb2, fma(cf.twice(4), dm1, cf(25) * dm2), gdm1);
+        gdm2 = fma(gb2, fma(cf(25), dm1, cf.twice(5) * dm2), gdm2);
     }
 
     // After face o (centre J): d[J-2] is complete, so is cell J-2; returns
     // cell J-3 (= o) and advances to face o+1 with cell J+3 = n.
     __device__ __forceinline__ double advance(const MarchArgs& a, double n) {
-        return advance([&](March64& w) { w.push(a, n); }, n);
+        return advance([&](March64& w) { w.push(a, n); });
     }
     // row: the row of face o + 1 in the table
     __device__ __forceinline__ double advance(const MarchArgs& a, const double* row, double n) {
-        return advance([&](March64& w) { w.push(a, VjpPair{row}, n); }, n);
+        return advance([&](March64& w) { w.push(a, VjpPair{row}, n); });
     }
     template <class Push>
-    __device__ __forceinline__ double advance(const Push& push, double n) {
+    __device__ __forceinline__ double advance(const Push& push) {
         gcm1 += gdm2;
         gcm2 -= gdm2;
         const double out = gcm3;
-        const double ne2 = (n - f.vp2) - f.dp1;
-        double c1, c2;
-        mm64_grad(f.e2, ne2, c1, c2);
         push(f);
-        cA1 = cB1; cA2 = cB2; cB1 = c1; cB2 = c2;
         gdm2 = gdm1; gdm1 = gd0; gd0 = gdp1; gdp1 = 0.0;
         gcm3 = gcm2; gcm2 = gcm1; gcm1 = gc0; gc0 = gcp1; gcp1 = 0.0;
         return out;
@@ -370,10 +371,13 @@ __device__ __forceinline__ void route_side(bool left, int code, double g, const 
     }
 }
 
+// SEG: columns in segments; whole columns have kernels of their own, as the
+// segment's bounds cost them registers (us per x/y/z gradient of whole columns,
+// 128^3 x 5: JS 802 with the bounds, 791 without, TENO 866 and 849).
 // PF: coefficients from the per-face table `tab` of `rows` rows (with LDR,
 // for every layout), which each CTA copies to shared memory: 28 doubles a
 // face, read at warp-uniform addresses.
-template <bool MPF, int KIND, bool TENOW, bool LDR, bool PF>
+template <bool MPF, int KIND, bool TENOW, bool LDR, bool PF, bool SEG>
 __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     vjp_march_kernel(const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tgL,
                      const __grid_constant__ CUtensorMap tgR, const __grid_constant__ CUtensorMap tgo,
@@ -511,7 +515,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     // the pull-back of face o, and the step to face o + 1 with cell n
     auto face = [&](MarchVjp& m, int o, double gL, double gR, int& pk, bool& ok) {
         if constexpr (PF) m.template face<MPF, TENOW, LDR>(a, VjpRow(rows + o * kVjpRow), gL, gR, pk, ok);
-        else m.template face<MPF, TENOW, LDR>(a, VjpParam{a}, gL, gR, pk, ok);
+        else m.template face<MPF, TENOW, LDR>(a, VjpParam{a, t.b2}, gL, gR, pk, ok);
     };
     auto advance = [&](MarchVjp& m, int o, double n) -> double {
         if constexpr (PF) return m.advance(a, rows + (o + 1) * kVjpRow, n);
@@ -519,8 +523,8 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
     };
 
     for (long long item = (long long)blockIdx.x * kVjpWarps + warp; item < a.n_items && !failed; item += nwarps) {
-        const int sg = (int)(item % a.n_seg);
-        long long tt = item / a.n_seg;
+        const int sg = SEG ? (int)(item % a.n_seg) : 0;
+        long long tt = SEG ? item / a.n_seg : item;
         int u0 = 0, wv = 0, vv = 0, c_end = 32;
         bool live;
         long long u, wl, vl;
@@ -558,7 +562,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
         // chunks [cs, ce) are written; a segment starts one chunk early, whose
         // faces reach its first cells
         const int n_all = (ns + 1) / F + 1;     // chunks until cell ns+5 is out
-        const int cs = sg * a.seg, ce = cs + a.seg < n_all ? cs + a.seg : n_all;
+        const int cs = SEG ? sg * a.seg : 0, ce = SEG && cs + a.seg < n_all ? cs + a.seg : n_all;
         const int cb = cs > 0 ? cs - 1 : 0;
         const int nch = ce - cb;
         const int ntiles = nch + 1;
@@ -620,7 +624,7 @@ __global__ void __launch_bounds__(kVjpWarps * 32, 1)
             const unsigned kc = k0 + c;
             if (!wait_stage(kc + 1)) { failed = true; break; }
             const int f0 = 4 + F * (cb + c);
-            const bool emit = cb + c >= cs;
+            const bool emit = !SEG || cb + c >= cs;
             if constexpr (KIND == 0 && !LDR) {
                 if (n_out >= 1) {
                     if (lane == 0) bulk_wait_read0();
@@ -794,6 +798,7 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
     t.acc = acc ? 1 : 0;
     t.gLp = gL;
     t.gRp = gR;
+    for (int k = 0; k < 6; ++k) t.b2[k] = ucf ? 2.0 * ucf[vjp_square(k)] : 0.0;
     cuuint64_t dims[4], strides[3];
     cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
     if (!folded) {
@@ -853,14 +858,19 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
     const size_t smem = (size_t)t.rows * kVjpRow * 8 + 1024 + (size_t)kVjpWarps * t.warp_bytes + (size_t)kVjpWarps * kVjpStages * 8;
     using KFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, VjpMarchArgs,
                          double*);
-#define WSB_VJP_ROW(MPF, TENOW)                                                      \
-    {{vjp_march_kernel<MPF, 0, TENOW, false, false>, vjp_march_kernel<MPF, 1, TENOW, false, false>}, \
-     {vjp_march_kernel<MPF, 0, TENOW, true, false>, vjp_march_kernel<MPF, 1, TENOW, true, false>},   \
-     {vjp_march_kernel<MPF, 0, TENOW, true, true>, vjp_march_kernel<MPF, 1, TENOW, true, true>}}
-    static const KFn table[2][2][3][2] = {{WSB_VJP_ROW(false, false), WSB_VJP_ROW(true, false)},
+    // the occupancy is that of one CTA per SM for every kernel
+    // (its registers), so the cut comes first and picks the kernel
+    vjp_march_cut(a, tma ? (long long)a.n_ut * a.Nw * a.NV : (a.n_cols + 31) / 32, (long long)sms * kVjpWarps);
+#define WSB_VJP_ROW(MPF, TENOW)                                                                                    \
+    {{vjp_march_kernel<MPF, 0, TENOW, false, false, false>, vjp_march_kernel<MPF, 1, TENOW, false, false, false>}, \
+     {vjp_march_kernel<MPF, 0, TENOW, false, false, true>, vjp_march_kernel<MPF, 1, TENOW, false, false, true>},   \
+     {vjp_march_kernel<MPF, 0, TENOW, true, false, true>, vjp_march_kernel<MPF, 1, TENOW, true, false, true>},     \
+     {vjp_march_kernel<MPF, 0, TENOW, true, true, true>, vjp_march_kernel<MPF, 1, TENOW, true, true, true>}}
+    static const KFn table[2][2][4][2] = {{WSB_VJP_ROW(false, false), WSB_VJP_ROW(true, false)},
                                           {WSB_VJP_ROW(false, true), WSB_VJP_ROW(true, true)}};
 #undef WSB_VJP_ROW
-    const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][tma ? 0 : (tab ? 2 : 1)][kind1 ? 1 : 0];
+    const int form = tma ? (a.n_seg > 1 ? 1 : 0) : (tab ? 3 : 2);
+    const KFn kfn = table[wp.scheme == TENO ? 1 : 0][mp ? 1 : 0][form][kind1 ? 1 : 0];
     // always the same limit: the size differs from call to call, and another
     // thread's call must not lower it between here and the launch
     int occ = 0;
@@ -869,9 +879,7 @@ inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, b
         cudaGetLastError();
         return 1003;
     }
-    const long long cap = (long long)sms * occ;
-    vjp_march_cut(a, tma ? (long long)a.n_ut * a.Nw * a.NV : (a.n_cols + 31) / 32, cap * kVjpWarps);
-    const long long blocks = std::min((a.n_items + kVjpWarps - 1) / kVjpWarps, cap);
+    const long long blocks = std::min((a.n_items + kVjpWarps - 1) / kVjpWarps, (long long)sms * occ);
     kfn<<<(unsigned)blocks, kVjpWarps * 32, smem, st>>>(mv, mL, mR, mo, ms, a, t, gv);
     return 0;
 }
