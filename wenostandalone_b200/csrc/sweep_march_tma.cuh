@@ -178,9 +178,9 @@ __device__ __forceinline__ void march_redo(const MarchArgs& a, const float* col,
 // One sweep of a grouped launch (sweep_march_tma_multi_kernel): its maps,
 // its arguments, and its first work item within the launch.  The sweeps of
 // a group share the kernel instance (order, weights, storage, tile kind,
-// MP), the coefficients (the kernel's MarchArgs) and the shared-memory
-// layout (the kernel's MarchTmaArgs); extents, strides, pointers, map axes,
-// loader and store kind are the entry's.
+// MP, TMA or per-lane loads and plain stores), the coefficients (the kernel's
+// MarchArgs) and the shared-memory layout (the kernel's MarchTmaArgs);
+// extents, strides, pointers and map axes are the entry's.
 // The part of a sweep's arguments a grouped work item reads outside the
 // face body; each item copies it (with the sweep's MarchTmaArgs) into its
 // warp's slot of shared memory, so the chunk loop reads it from there
@@ -355,8 +355,8 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
             }
             __syncwarp();
         }
-        // geometry, maps, loader and store kind of this item's sweep; the
-        // sweep's full arguments for the faces redone by the reference sequence
+        // geometry and maps of this item's sweep; the sweep's full arguments for
+        // the faces redone by the reference sequence
         const auto& g = mtma_geo_of<MULTI>(a, slot);
         const MarchTmaArgs& te = MULTI ? slot->ia.t : t;
         // (grouped: read from the slot where used)
@@ -877,8 +877,7 @@ inline void march_segments(MarchArgs& a, int order, bool pst, long long seg_face
     a.n_items = cols * a.n_seg;
 }
 
-// Shared-memory layout of the plan's kernel (pst: the single-sweep kernels
-// with plain stores).
+// Shared-memory layout of the plan's kernel (pst: with plain stores).
 template <typename T>
 void march_layout(MtmaPlan& P, int order, bool pst) {
     MarchTmaArgs& t = P.t;
@@ -987,7 +986,9 @@ int plan_march_tma(const long long E[3], const SweepGeom& g, int dir, bool folde
 // paths 0 TMA tiles in and out, 1 per-lane loads and TMA stores, 2 per-lane
 // loads and plain stores.  Per-lane loads read any alignment, so path 2
 // serves every layout the others refuse.  PF: with the per-face table, whose
-// kernels load by TMA (path 0) or take path 2.
+// kernels load by TMA (path 0) or take path 2.  (Path 0 has no row tiles of
+// floats: the field's rows are 6 longer than the face rows, so never both
+// multiples of 4.)
 using MtmaFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MarchArgs, MarchTmaArgs);
 template <typename T, bool PF, int ORDER, int WS, bool MPF, int KIND>
 MtmaFn mtma_path(int path) {
@@ -997,7 +998,10 @@ MtmaFn mtma_path(int path) {
     if constexpr (!PF) {
         if (path == 1) return sweep_march_tma_kernel<MPF, KIND, T, 1, false, ORDER, WS>;
     }
-    return path == 0 ? sweep_march_tma_kernel<MPF, KIND, T, 0, PF, ORDER, WS> : nullptr;
+    if constexpr (KIND == 1 || sizeof(T) == 8) {
+        if (path == 0) return sweep_march_tma_kernel<MPF, KIND, T, 0, PF, ORDER, WS>;
+    }
+    return nullptr;
 }
 template <typename T, bool PF, int ORDER, int WS>
 MtmaFn mtma_pick(bool mp, bool kind1, int path) {
@@ -1067,11 +1071,14 @@ int launch_march_tma(const long long E[3], const SweepGeom& g, int dir, bool fol
 using MtmaMultiFn = void (*)(const MtmaEntry*, const long long*, int, long long, MarchArgs, MarchTmaArgs);
 template <typename T, int ORDER, int WS, bool PST>
 MtmaMultiFn mtma_multi_pick(bool mp, bool kind1) {
-    static const MtmaMultiFn tab[2][2] = {{sweep_march_tma_multi_kernel<false, 0, T, ORDER, WS, PST>,
-                                           sweep_march_tma_multi_kernel<false, 1, T, ORDER, WS, PST>},
-                                          {sweep_march_tma_multi_kernel<true, 0, T, ORDER, WS, PST>,
-                                           sweep_march_tma_multi_kernel<true, 1, T, ORDER, WS, PST>}};
-    return tab[mp ? 1 : 0][kind1 ? 1 : 0];
+    if (kind1)
+        return mp ? sweep_march_tma_multi_kernel<true, 1, T, ORDER, WS, PST>
+                  : sweep_march_tma_multi_kernel<false, 1, T, ORDER, WS, PST>;
+    // (row tiles of floats have plain stores, see mtma_path)
+    if constexpr (PST || sizeof(T) == 8)
+        return mp ? sweep_march_tma_multi_kernel<true, 0, T, ORDER, WS, PST>
+                  : sweep_march_tma_multi_kernel<false, 0, T, ORDER, WS, PST>;
+    return nullptr;
 }
 template <typename T, bool PST>
 MtmaMultiFn mtma_multi_kernel(int order, bool teno, bool mp, bool kind1) {

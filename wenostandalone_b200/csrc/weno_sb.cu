@@ -631,8 +631,8 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
 //          time-first on the entries' estimated cost, so small blocks run
 //          beside each other and beside the tails of large ones.
 //  mode 2: the entries that a marching engine covers are grouped by kernel
-//          instance (storage, order, weights, MP, tile kind) and
-//          coefficients; each group is one launch of the grouped TMA
+//          instance (storage, order, weights, MP, tile kind, TMA or
+//          plain loads and stores) and coefficients; each group is one launch of the grouped TMA
 //          marching kernel over the work items of all its sweeps (columns
 //          cut into segments of about `seg_faces` faces), the groups spread
 //          over `branches` graph branches by longest-processing-time-first;
