@@ -368,6 +368,7 @@ def run_ours(args):
     # FP32-bulk variant (same sweeps, FP32 v_rs_ws field and face states)
     fp32 = None
     if not args.no_extras and not fp32_main:
+        step()  # (the per-face step left the states of other coefficients)
         fp32 = measure_fp32_bulk(g, v, faces, outs, stream, K, dev)
         drop = measure_drop_in(g, v, faces, outs, stream, K, dev)
     else:
