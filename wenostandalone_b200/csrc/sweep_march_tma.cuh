@@ -1,7 +1,8 @@
 // sweep_march_tma.cuh -- the marching sweep (sweep_march.cuh engines: WENO3
 // / WENO5 / WENO7, JS or TENO weights, FP64 or FP32-bulk, face-independent
-// coefficients or, FP64 WENO5-JS, a per-face table) with TMA staging of its
-// input cells and output face states.
+// coefficients or, in FP64, a per-face table) with TMA staging of its input
+// cells and output face states, or per-lane copies and plain stores for
+// layouts that TMA refuses.
 //
 // The marching kernel of sweep_march.cuh spends, at 200^3 x 8, about as
 // much time waiting on its per-lane global loads (a few cells ahead in
@@ -832,9 +833,9 @@ __global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST>
 // states leave by TMA stores when the face rows (ns elements) are 16-byte
 // multiples from 16-byte aligned bases, else by plain stores from the same
 // staging tiles.  seg_faces > 0 cuts every column into segments of about
-// that many faces; 0 sizes the segments for `sms` SMs (march_segments).  Returns 1003 (unsupported) for sweeps of
-// fewer than 8 faces, a lane axis the march arguments did not choose, or a
-// missing driver entry point.
+// that many faces; 0 sizes the segments for `sms` SMs (march_segments).
+// Returns 1003 (unsupported) for sweeps of fewer than 8 faces, a lane axis the
+// march arguments did not choose, or a missing driver entry point.
 struct MtmaPlan {
     CUtensorMap mi, mL, mR;
     MarchArgs a;

@@ -43,7 +43,10 @@
 // sweep (27 coefficients a face) in shared memory, read at warp-uniform
 // addresses; staged per chunk and warp it would not fit beside the tiles.
 // us per x/y/z gradient, 97x80x65 x 5: 689 with one thread per column
-// (vjp_kernel), 561 here.  Bound by FP64 issue with 8 warps an SM.
+// (vjp_kernel), 561 here.  Bound by latency with 8 warps an SM (issue slots
+// 40%, FP64 pipe 32%, against 57% and 56% without the table and aligned):
+// dependent uses, the rows' shared loads, instruction fetch, and a last round
+// of the resident warps that is 11% (y) and 32% (z) full.
 #pragma once
 
 #include <cuda.h>
@@ -64,7 +67,7 @@ struct VjpMarchArgs {
     int acc;            // add to the gradient already in gv
     int vbytes;         // one v (or old-gradient) tile
     int stage_bytes;    // v (and old gradient) tiles of one stage
-    int warp_bytes;     // multiple of 1024
+    int warp_bytes;     // multiple of 512
     unsigned tx_bytes;  // bytes one stage receives
     const double* gLp;  // cotangents (ns, c1, c2, V)
     const double* gRp;
@@ -766,13 +769,6 @@ inline void vjp_march_cut(MarchArgs& a, long long tiles, long long warps) {
     a.n_items = tiles * a.n_seg;
 }
 
-// Host side: the marching adjoint for FP64 WENO5 with JS or TENO weights and
-// face-independent coefficients (ucf), or with the per-face table tab built
-// from cp (the lanes then load in every layout).  TMA staging when every base
-// and row is a 16-byte multiple, copies by the lanes otherwise.  Returns 1003
-// (unsupported) for sweeps of fewer than 8 faces or a lane axis the march arguments did not choose; the caller then
-// runs vjp_kernel.  gv must already hold what is to be added to when acc is
-// set.
 // Rows of the per-face table (the last chunk's last face reads the pairs of
 // three rows after its own), and the most for which it fits into shared
 // memory beside the warps' tiles (227 KB in all: sweeps of up to 214 faces);
@@ -782,6 +778,13 @@ inline long long vjp_table_rows(const SweepGeom& g) { return (g.ns + 1) / kTmaF 
 constexpr int kVjpLdrWarpBytes = (kVjpStages * (4096 + 2048) + 13 * 32 * 8 + 3 * 32 * 8 + 511) / 512 * 512;
 constexpr long long kVjpMaxRows =
     (kVjpMaxSmem - 1024 - kVjpWarps * (kVjpLdrWarpBytes + kVjpStages * 8)) / (kVjpRow * 8);
+// Host side: the marching adjoint for FP64 WENO5 with JS or TENO weights and
+// face-independent coefficients (ucf), or with the per-face table tab built
+// from cp (the lanes then load in every layout).  TMA staging when every base
+// and row is a 16-byte multiple, copies by the lanes otherwise.  Returns 1003
+// (unsupported) for sweeps of fewer than 8 faces or a lane axis the march
+// arguments did not choose; the caller then runs vjp_kernel.  gv must already
+// hold what is to be added to when acc is set.
 inline int launch_vjp_march(const long long E[3], const SweepGeom& g, int dir, bool folded, bool mp, bool acc,
                             const double* v, const double* ucf, const double* tab, const CoefPtrs& cp,
                             const WenoParams& wp, const double* gL, const double* gR, double* gv, cudaStream_t st,

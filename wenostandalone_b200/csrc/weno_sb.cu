@@ -584,7 +584,7 @@ int launch_vjp(const Dims& d, const weno_sb_grid* gr, int dir, int order, unsign
         if (rc != WENO_SB_ERR_UNSUPPORTED) return rc == 0 ? cuda_err(cudaGetLastError(), "vjp march launch") : rc;
     }
     // coefficient arrays: the marching adjoint with a per-face table, where it
-    // fits (us per x/y/z gradient, 97x80x65 x 5: 574; vjp_kernel 689), but not
+    // fits (us per x/y/z gradient, 97x80x65 x 5: 561; vjp_kernel 689), but not
     // into a stream capture, where the table would be memory of the graph
     if (!uni && order == 5 && (gr->scheme == WENO_SB_JS || teno) && kernel_choice() != 1 &&
         a.g.ns >= 8 && vjp_table_rows(a.g) <= kVjpMaxRows && !capturing(st)) {
