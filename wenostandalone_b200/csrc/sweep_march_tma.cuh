@@ -89,8 +89,9 @@ __host__ __device__ constexpr int mtma_outs(bool pf, bool pst, int order, int es
 // engine for WENO3-JS and for TENO weights, which the one-thread-per-face
 // kernels computed in FP64 before, with one rounding.  us per sweep of 163
 // cells, 125 x 151 columns x 8, on those kernels / with the FP32 engine (whose
-// weights and sums are FP32) / here: WENO3 240 / 135 / 193, WENO5-TENO 856 /
-// 207 / 262, WENO7-TENO 2250 / 277 / 385.
+// weights and sums are FP32) / here: WENO3 240 / 135 / 176 (four CTAs per SM
+// at 128 registers, 24 bytes spilled; three at 162: 193), WENO5-TENO 856 / 207
+// / 262, WENO7-TENO 2250 / 277 / 385.
 __host__ __device__ constexpr bool mtma_wide(bool pst, int order, int ws, int es) {
     return pst && es == 4 && (order == 3 || ws == 3);
 }
@@ -792,19 +793,17 @@ __device__ __forceinline__ void march_tma_body(const CUtensorMap* tin0, const CU
 #ifndef WSB_MTMA_MIN_BLOCKS_W7
 #define WSB_MTMA_MIN_BLOCKS_W7 2  // WENO7 carries ~27 doubles of state: 3 CTAs per SM would spill
 #endif
-// CTAs per SM by order (WENO3: 4, but 3 with plain stores from the FP64
-// engine: its second output tile leaves no shared memory for a fourth, and
-// storing FP32 its registers do not fit)
-template <int ORDER, typename T, bool PST, bool E64 = sizeof(T) == 8>
+// CTAs per SM by order (WENO3: 4, but 3 for plain stores of FP64, whose second
+// output tile leaves no shared memory for a fourth)
+template <int ORDER, typename T, bool PST>
 constexpr int kMtmaMinBlocks = ORDER == 7 ? WSB_MTMA_MIN_BLOCKS_W7
-                               : ORDER == 3 && !(PST && E64)
+                               : ORDER == 3 && !(PST && sizeof(T) == 8)
                                    ? 4
                                    : (sizeof(T) == 8 ? WSB_MTMA_MIN_BLOCKS : WSB_MTMA_MIN_BLOCKS_F32);
 
 // One sweep: maps and arguments in the parameter bank.
 template <bool MPF, int KIND, typename T, int LDR, bool PF, int ORDER = 5, int WS = 0, bool PST = false>
-__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST, sizeof(T) == 8 ||
-                                                                  mtma_wide(PST, ORDER, WS, (int)sizeof(T))>))
+__global__ void __launch_bounds__(kTmaWarps * 32, (kMtmaMinBlocks<ORDER, T, PST>))
     sweep_march_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap toutL,
                            const __grid_constant__ CUtensorMap toutR, const __grid_constant__ MarchArgs a,
                            const MarchTmaArgs t) {
